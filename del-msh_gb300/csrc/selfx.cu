@@ -2,11 +2,11 @@
 // (trimesh3_intersection.rs:1-179: search_with_bvh_inside_branch and
 // search_with_bvh_between_branches).  The recursion inside(root) visits, at
 // every branch n, between(left(n), right(n)) and recurses; so the pairs are
-// exactly the union over branches n of between(left(n), right(n)).  Each
-// start pair is searched depth-first by one thread with an explicit stack of
-// node pairs, in rounds: a thread that has visited kBudget pairs hands its
-// remaining stack to the next round, so that the few large subtree pairs
-// near the root spread over many threads instead of one.
+// exactly the union over branches n of between(left(n), right(n)).  Warps
+// take start pairs and search them 32 node pairs at a time from a stack in
+// shared memory, in rounds: a warp that still has pairs when the round's start
+// pairs have run out hands them to the next round, so that the few large
+// subtree pairs near the root spread over all warps instead of one.
 // Every unordered pair of leaves meets at exactly one branch (their
 // lowest common ancestor), with the triangle of the left subtree first, as
 // in the recursion; only the order of the output list differs.
@@ -31,7 +31,6 @@ namespace dm {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kPairStack = 192;  // node pairs on the per-thread stack
 
 __device__ __forceinline__ float3 lerp_cross(float3 vi, float3 vj, float di, float dj) {
   const float s = __fdiv_rn(di, __fsub_rn(di, dj));
@@ -157,8 +156,25 @@ __device__ __forceinline__ bool tri_pair(const MeshView& m, uint32_t it, uint32_
   return false;
 }
 
-__device__ __forceinline__ bool boxes_overlap(const float* a, const float* b) {
-  return a[0] <= b[3] && b[0] <= a[3] && a[1] <= b[4] && b[1] <= a[4] && a[2] <= b[5] && b[2] <= a[5];
+struct Box6 {
+  float2 a, b, c;  // lo.x lo.y | lo.z hi.x | hi.y hi.z
+};
+
+// kVec: the box array is 8-byte aligned, as boxes of 24 bytes then are.
+template <bool kVec>
+__device__ __forceinline__ Box6 load_box(const float* aabb, uint32_t n) {
+  const float* f = aabb + static_cast<size_t>(n) * 6;
+  if constexpr (kVec) {
+    const float2* p = reinterpret_cast<const float2*>(f);
+    return Box6{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+  } else {
+    return Box6{make_float2(__ldg(f), __ldg(f + 1)), make_float2(__ldg(f + 2), __ldg(f + 3)),
+                make_float2(__ldg(f + 4), __ldg(f + 5))};
+  }
+}
+
+__device__ __forceinline__ bool overlap6(const Box6& p, const Box6& q) {
+  return p.a.x <= q.b.y && q.a.x <= p.b.y && p.a.y <= q.c.x && q.a.y <= p.c.x && p.b.x <= q.c.y && q.b.x <= p.c.y;
 }
 
 __device__ __forceinline__ void report_pair(const MeshView& m, uint32_t a0, uint32_t b0, uint32_t capacity,
@@ -178,114 +194,282 @@ __device__ __forceinline__ void report_pair(const MeshView& m, uint32_t a0, uint
   sg[5] = p1.z;
 }
 
-// The first round starts from (left(n), right(n)) for every branch n.
-__global__ void __launch_bounds__(kThreads) k_selfx_init(MeshView m, uint2* frontier) {
-  const uint32_t n = blockIdx.x * kThreads + threadIdx.x;
-  if (m.num_tri < 2 || n >= m.num_tri - 1) return;
-  frontier[n] = make_uint2(__ldg(m.bvhnodes + static_cast<size_t>(n) * 3 + 1),
-                           __ldg(m.bvhnodes + static_cast<size_t>(n) * 3 + 2));
-}
+// One warp searches with one stack of node pairs in shared memory: each step
+// pops up to 32 pairs, one per lane, and pushes the child pairs whose boxes
+// overlap.  A pair of leaves goes to a small buffer, tested 32 at a time, so
+// that the long triangle test never runs for a few lanes.  What bounds it is
+// the dependent round trips of a step (records, then boxes), hidden by the 32
+// resident warps per SM.  A search by single threads, each with a stack of its
+// own in local memory, ran eight rounds of 500 us whose ends were a few long
+// threads: 4.24 ms for two crossing tori of 260,084 triangles in all, against
+// 0.33 ms for the four rounds here.
+constexpr uint32_t kWarpsPerBlock = kThreads / 32;
+constexpr uint32_t kPairStack = 704;   // node pairs on a warp's stack
+constexpr uint32_t kLeafBuffer = 64;   // leaf pairs waiting for their test
+// Every so many steps a warp looks whether the round's start pairs are all
+// given out; if so warps are running idle, and it hands its own pairs to the
+// next round, where they are dealt out anew.  The subtree pairs near the root,
+// which hold most of the work, are split this way.  The whole query with its Python
+// side took 1.49, 1.18, 1.03 and 1.08 ms for 8, 16, 32 and 64 steps.
+constexpr uint32_t kRoundSteps = 32;
 
-// One round: each thread searches depth-first from one start pair with an
-// explicit stack; after kBudget node-pair visits it hands its remaining stack
-// to the next round (when all of it fits there; otherwise it finishes alone),
-// so that the few large subtree pairs near the root are split over many
-// threads in the following rounds.
-constexpr uint32_t kBudget = 512;
+constexpr uint32_t kAloneLooks = 2048, kAloneMost = 1u << 17;  // looks of a search that nothing ends
 
-__global__ void __launch_bounds__(kThreads) k_selfx_round(MeshView m, const uint2* __restrict__ start,
-                                                         uint32_t num_start, uint2* next, uint32_t* num_next,
-                                                         uint64_t next_cap, uint32_t capacity, uint32_t* pairs,
-                                                         float* segments, uint32_t* count, uint32_t* status) {
-  const uint32_t k = blockIdx.x * kThreads + threadIdx.x;
-  if (k >= num_start) return;
-  const uint32_t num_node = 2 * m.num_tri - 1;
-  const uint32_t* bn = m.bvhnodes;
-  uint2 stack[kPairStack];
-  int sp = 0;
-  stack[sp++] = start[k];
-  uint32_t visits = 0;
-  while (sp > 0) {
-    if (++visits > kBudget && sp > 1) {
-      // reserve room only if the whole stack fits, so that the next round's
-      // list has no unwritten holes (a bounded number of attempts)
-      uint32_t cur = *reinterpret_cast<volatile uint32_t*>(num_next);
-      bool handed = false;
-      for (int attempt = 0; attempt < 64 && cur + static_cast<uint64_t>(sp) <= next_cap; ++attempt) {
-        const uint32_t seen = atomicCAS(num_next, cur, cur + static_cast<uint32_t>(sp));
-        if (seen == cur) {
-          for (int q = 0; q < sp; ++q) next[cur + q] = stack[q];
-          handed = true;
-          break;
-        }
-        cur = seen;
+// A round's start pairs are `start[0 .. *num_start)`, or without a list the
+// children (left(n), right(n)) of every branch n.
+struct RoundList {
+  const uint2* start;
+  const uint32_t* num_start;
+  uint32_t* take;      // start pairs given out
+  uint2* next;         // the next round's list
+  uint32_t* num_next;
+  uint32_t next_cap;
+};
+
+// Moves the `k` bottom pairs of the stack to the next round's list if they all
+// fit there.
+__device__ __forceinline__ bool hand_over(const RoundList& rl, uint2* stack, uint32_t& sp, uint32_t k, uint32_t lane) {
+  uint32_t at = 0, ok = 0;
+  if (lane == 0) {
+    // a reservation that would pass the end is refused by compare-and-swap, so
+    // that the list has no unwritten holes (a bounded number of attempts)
+    uint32_t cur = *reinterpret_cast<volatile uint32_t*>(rl.num_next);
+    for (int attempt = 0; attempt < 64 && cur <= rl.next_cap && k <= rl.next_cap - cur; ++attempt) {
+      const uint32_t seen = atomicCAS(rl.num_next, cur, cur + k);
+      if (seen == cur) {
+        at = cur;
+        ok = 1;
+        break;
       }
-      if (handed) return;
-      visits = 0;  // no room: keep going alone
-    }
-    const uint2 pr = stack[--sp];
-    if (pr.x >= num_node || pr.y >= num_node) {
-      raise_status(status, kStatusBadIndex);
-      continue;
-    }
-    if (!boxes_overlap(m.aabb + static_cast<size_t>(pr.x) * 6, m.aabb + static_cast<size_t>(pr.y) * 6)) continue;
-    const uint32_t a0 = __ldg(bn + static_cast<size_t>(pr.x) * 3 + 1), a1 = __ldg(bn + static_cast<size_t>(pr.x) * 3 + 2);
-    const uint32_t b0 = __ldg(bn + static_cast<size_t>(pr.y) * 3 + 1), b1 = __ldg(bn + static_cast<size_t>(pr.y) * 3 + 2);
-    const bool la = a1 == kUMax, lb = b1 == kUMax;
-    if (la && lb) {
-      report_pair(m, a0, b0, capacity, pairs, segments, count, status);
-      continue;
-    }
-    const int need = (!la && !lb) ? 4 : 2;
-    if (sp + need > kPairStack) {
-      raise_status(status, kStatusStackOverflow);
-      return;
-    }
-    // pushed in reverse of the recursion's order, which it then follows
-    if (!la && !lb) {
-      stack[sp++] = make_uint2(a1, b1);
-      stack[sp++] = make_uint2(a0, b1);
-      stack[sp++] = make_uint2(a1, b0);
-      stack[sp++] = make_uint2(a0, b0);
-    } else if (!la) {
-      stack[sp++] = make_uint2(a1, pr.y);
-      stack[sp++] = make_uint2(a0, pr.y);
-    } else {
-      stack[sp++] = make_uint2(pr.x, b1);
-      stack[sp++] = make_uint2(pr.x, b0);
+      cur = seen;
     }
   }
+  at = __shfl_sync(0xffffffffu, at, 0);
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  if (!ok) return false;
+  for (uint32_t q = lane; q < k; q += 32) rl.next[at + q] = stack[q];
+  __syncwarp();
+  // the rest moves down, 32 pairs at a time (each read before it is overwritten)
+  for (uint32_t q = k; q < sp; q += 32) {
+    const uint2 v = q + lane < sp ? stack[q + lane] : make_uint2(0, 0);
+    __syncwarp();
+    if (q + lane < sp) stack[q + lane - k] = v;
+    __syncwarp();
+  }
+  sp -= k;
+  return true;
+}
+
+template <bool kVec>
+__global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundList rl, uint32_t capacity,
+                                                            uint32_t* pairs, float* segments, uint32_t* count,
+                                                            uint32_t* status) {
+  __shared__ uint2 sh_stack[kWarpsPerBlock][kPairStack];
+  __shared__ uint2 sh_leaf[kWarpsPerBlock][kLeafBuffer];
+  constexpr uint32_t kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  uint2* stack = sh_stack[warp];
+  uint2* leaf = sh_leaf[warp];
+  const uint32_t num_node = 2 * m.num_tri - 1;
+  const uint32_t num_start = rl.start ? *rl.num_start : m.num_tri - 1;
+  // start pairs are dealt out a few at a time (8 against 32: 0.95 against 1.03 ms,
+  // as fewer warps end with much left), and one by one when there are few
+  const uint32_t chunk = min(8u, max(1u, num_start / (gridDim.x * kWarpsPerBlock)));
+  uint32_t sp = 0, nleaf = 0, steps = 0, alone = 0;
+  bool more = num_start > 0, bad = false;
+  for (;;) {
+    bool live = false;  // this lane holds a pair of branches, or of a branch and a leaf
+    uint32_t a = 0, b = 0, a0 = 0, a1 = 0, b0 = 0, b1 = 0;
+    if (more && sp < chunk) {
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(rl.take, chunk);
+      base = __shfl_sync(kAll, base, 0);
+      if (base >= num_start || base + chunk < base) {
+        more = false;
+        continue;
+      }
+      bool mine = lane < chunk && base + lane < num_start;
+      if (mine) {
+        if (rl.start) {
+          const uint2 pr = rl.start[base + lane];
+          a = pr.x;
+          b = pr.y;
+        } else {
+          a = __ldg(m.bvhnodes + static_cast<size_t>(base + lane) * 3 + 1);
+          b = __ldg(m.bvhnodes + static_cast<size_t>(base + lane) * 3 + 2);
+        }
+        if (a >= num_node || b >= num_node) {
+          bad = true;
+          mine = false;
+        }
+      }
+      const bool keep = mine && overlap6(load_box<kVec>(m.aabb, a), load_box<kVec>(m.aabb, b));
+      const uint32_t mask = __ballot_sync(kAll, keep);
+      if (keep) stack[sp + __popc(mask & lt)] = make_uint2(a, b);
+      sp += __popc(mask);  // sp < chunk <= 32 before, so there is room
+      __syncwarp();
+      continue;
+    }
+    if (sp == 0) break;
+    if (steps >= kRoundSteps) {
+      steps = 0;
+      // while start pairs are left no warp is idle, and there is nothing to
+      // split; a search of this length without an end (a tree with a cycle,
+      // for which the rounds are the bound) is handed over all the same
+      uint32_t taken = 0;
+      if (lane == 0) taken = *reinterpret_cast<volatile uint32_t*>(rl.take);
+      taken = __shfl_sync(kAll, taken, 0);
+      if ((taken >= num_start || alone >= kAloneLooks) && hand_over(rl, stack, sp, sp, lane)) {
+        alone = 0;
+        continue;
+      }
+      if (++alone > kAloneMost) {  // no room in the list, and no end
+        if (lane == 0) raise_status(status, kStatusStackOverflow);
+        break;
+      }
+    }
+    ++steps;
+    // a popped pair leaves room for at most four: fewer are popped while the
+    // stack is nearly full, after handing its older half on if that fits
+    if (sp + 96 > kPairStack) hand_over(rl, stack, sp, sp / 2, lane);
+    const uint32_t room = (kPairStack - sp) / 3;
+    if (room == 0) {
+      if (lane == 0) raise_status(status, kStatusStackOverflow);
+      break;
+    }
+    const uint32_t k = min(min(32u, sp), room);
+    if (lane < k) {
+      const uint2 pr = stack[sp - 1 - lane];
+      a = pr.x;
+      b = pr.y;
+      const uint32_t* ra = m.bvhnodes + static_cast<size_t>(a) * 3;
+      const uint32_t* rb = m.bvhnodes + static_cast<size_t>(b) * 3;
+      a0 = __ldg(ra + 1);
+      a1 = __ldg(ra + 2);
+      b0 = __ldg(rb + 1);
+      b1 = __ldg(rb + 2);
+      live = true;
+    }
+    sp -= k;
+    __syncwarp();
+    const bool la = a1 == kUMax, lb = b1 == kUMax;
+    const uint32_t lmask = __ballot_sync(kAll, live && la && lb);
+    if (live && la && lb) {
+      leaf[nleaf + __popc(lmask & lt)] = make_uint2(a0, b0);
+      live = false;
+    }
+    nleaf += __popc(lmask);  // at most 31 before this step
+    // the two (or one) nodes on each side and the overlaps among them
+    bool push[4] = {false, false, false, false};
+    const uint32_t xa[2] = {la ? a : a0, a1}, xb[2] = {lb ? b : b0, b1};
+    if (live) {
+      if (xa[0] >= num_node || xb[0] >= num_node || (!la && a1 >= num_node) || (!lb && b1 >= num_node)) {
+        bad = true;
+        live = false;
+      }
+    }
+    if (live) {
+      const Box6 p0 = load_box<kVec>(m.aabb, xa[0]), q0 = load_box<kVec>(m.aabb, xb[0]);
+      const Box6 p1 = la ? p0 : load_box<kVec>(m.aabb, a1), q1 = lb ? q0 : load_box<kVec>(m.aabb, b1);
+      push[0] = overlap6(p0, q0);
+      push[1] = !la && overlap6(p1, q0);
+      push[2] = !lb && overlap6(p0, q1);
+      push[3] = !la && !lb && overlap6(p1, q1);
+    }
+    // pushed in reverse of the recursion's order
+#pragma unroll
+    for (int c = 3; c >= 0; --c) {
+      const uint32_t mask = __ballot_sync(kAll, push[c]);
+      if (push[c]) stack[sp + __popc(mask & lt)] = make_uint2(xa[c & 1], xb[c >> 1]);
+      sp += __popc(mask);
+    }
+    __syncwarp();
+    if (nleaf >= 32) {
+      nleaf -= 32;
+      const uint2 pr = leaf[nleaf + lane];
+      report_pair(m, pr.x, pr.y, capacity, pairs, segments, count, status);
+      __syncwarp();
+    }
+  }
+  if (lane < nleaf) {
+    const uint2 pr = leaf[lane];
+    report_pair(m, pr.x, pr.y, capacity, pairs, segments, count, status);
+  }
+  if (bad) raise_status(status, kStatusBadIndex);
+}
+
+}  // namespace
+
+namespace {
+
+constexpr uint32_t kRounds = 64;       // rounds between two clearings of the counters
+constexpr size_t kHeaderBytes = 1024;  // [start pairs given out, length of the list] per round
+
+int round_grid() {
+  static int cached[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (cached[dev] == 0) {
+    int sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_selfx_round<true>, kThreads, 0);
+    cached[dev] = (sms > 0 ? sms : 152) * (per_sm > 0 ? per_sm : 1);
+  }
+  return cached[dev];
 }
 
 }  // namespace
 
 size_t self_intersection_scratch_bytes(uint32_t num_tri) {
   const uint64_t cap = num_tri < (1u << 20) ? (1u << 20) : num_tri;  // start pairs per round
-  return 256 + 2 * cap * sizeof(uint2);
+  return kHeaderBytes + 2 * cap * sizeof(uint2);
 }
 
 int launch_self_intersection(cudaStream_t s, const MeshView& m, uint32_t capacity, uint32_t* pairs, float* segments,
                              uint32_t* count, void* scratch, size_t scratch_bytes, uint32_t* status) {
   if (m.num_tri < 2) return 0;
-  uint32_t* num_next = static_cast<uint32_t*>(scratch);
-  const uint64_t cap = (scratch_bytes - 256) / (2 * sizeof(uint2));
-  uint2* fa = reinterpret_cast<uint2*>(static_cast<char*>(scratch) + 256);
-  uint2* fb = fa + cap;
-  uint32_t num_cur = m.num_tri - 1;
-  k_selfx_init<<<(num_cur + kThreads - 1) / kThreads, kThreads, 0, s>>>(m, fa);
-  // rounds until no thread hands work on (each round either finishes its
-  // threads' work or splits it, so there are few; bounded here)
-  for (int round = 0; round < 1000 && num_cur > 0; ++round) {
-    if (cudaMemsetAsync(num_next, 0, sizeof(uint32_t), s) != cudaSuccess) return -1;
-    k_selfx_round<<<(num_cur + kThreads - 1) / kThreads, kThreads, 0, s>>>(m, fa, num_cur, fb, num_next, cap,
-                                                                           capacity, pairs, segments, count, status);
-    uint32_t n = 0;
-    if (cudaMemcpyAsync(&n, num_next, sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess) return -1;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
-    num_cur = n;  // every reservation was written in full
-    uint2* t = fa;
-    fa = fb;
-    fb = t;
+  uint32_t* counters = static_cast<uint32_t*>(scratch);  // 2 * kRounds words and the last list's length
+  static_assert((2 * kRounds + 2) * sizeof(uint32_t) <= kHeaderBytes, "counters");
+  const uint64_t cap = (scratch_bytes - kHeaderBytes) / (2 * sizeof(uint2));
+  uint2* list[2] = {reinterpret_cast<uint2*>(static_cast<char*>(scratch) + kHeaderBytes), nullptr};
+  list[1] = list[0] + cap;
+  int full = round_grid();
+  const uint32_t need = (m.num_tri - 1 + kThreads - 1) / kThreads;
+  if (cudaMemsetAsync(counters, 0, kHeaderBytes, s) != cudaSuccess) return -1;
+  // Rounds until no warp hands work on.  Each round either finishes its warps'
+  // work or splits it, so there are few (bounded here).  The length of a
+  // round's list stays on the device: kAhead rounds are launched between two
+  // looks at it, an empty one costs 2 us and a look 15.
+  constexpr uint32_t kAhead = 4;
+  for (uint32_t round = 0; round < 4000; ++round) {
+    const uint32_t r = round % kRounds;
+    if (r == 0 && round > 0) {  // the list's length moves to the front, the rest is cleared
+      if (cudaMemcpyAsync(counters + 1, counters + 2 * kRounds + 1, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s) !=
+              cudaSuccess ||
+          cudaMemsetAsync(counters + 2, 0, kHeaderBytes - 8, s) != cudaSuccess ||
+          cudaMemsetAsync(counters, 0, 4, s) != cudaSuccess)
+        return -1;
+    }
+    RoundList rl;
+    rl.take = counters + 2 * r;
+    rl.start = round == 0 ? nullptr : list[(round + 1) & 1];
+    rl.num_start = counters + 2 * r + 1;
+    rl.next = list[round & 1];
+    rl.num_next = counters + 2 * (r + 1) + 1;
+    rl.next_cap = static_cast<uint32_t>(cap < 0x7fffffffu ? cap : 0x7fffffffu);
+    // the first round of a small mesh has no more warps than start pairs
+    const int grid = round == 0 && need < static_cast<uint32_t>(full) ? static_cast<int>(need) : full;
+    if (reinterpret_cast<uintptr_t>(m.aabb) % 8 == 0)
+      k_selfx_round<true><<<grid, kThreads, 0, s>>>(m, rl, capacity, pairs, segments, count, status);
+    else
+      k_selfx_round<false><<<grid, kThreads, 0, s>>>(m, rl, capacity, pairs, segments, count, status);
+    if (round % kAhead == kAhead - 1) {
+      uint32_t n = 0;
+      if (cudaMemcpyAsync(&n, rl.num_next, sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess) return -1;
+      if (cudaStreamSynchronize(s) != cudaSuccess) return -1;
+      if (n == 0) return 0;
+    }
   }
   return 0;
 }
