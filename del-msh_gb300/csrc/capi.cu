@@ -671,7 +671,7 @@ int dm_pix2tri_by_raycast(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, u
   if (int e = sc.acquire(scratch, scratch_bytes, dm::cast_scratch_bytes(n, num_tri), s, nullptr)) return e;
   dm::CastScratch cs;
   dm::cast_scratch_carve(sc.ptr, n, num_tri, &cs);
-  DM_CUDA(cudaMemsetAsync(cs.counters, 0, 16, s));
+  DM_CUDA(cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, s));
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb};
   dm::CastOut o{pix2tri, pix2t, nullptr};
   dm::launch_cast_pixels(s, img_w, img_h, transform_ndc2world, m, o, cs, status_ptr());
@@ -693,7 +693,7 @@ int dm_search_bvh3_first_intersection_ray(uint64_t stream_ptr, uint32_t num_ray,
   if (int e = sc.acquire(scratch, scratch_bytes, dm::cast_scratch_bytes(num_ray, num_tri), s, nullptr)) return e;
   dm::CastScratch cs;
   dm::cast_scratch_carve(sc.ptr, num_ray, num_tri, &cs);
-  DM_CUDA(cudaMemsetAsync(cs.counters, 0, 16, s));
+  DM_CUDA(cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, s));
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb};
   dm::CastOut o{hit_tri, hit_t, hit_bc};
   dm::launch_cast_rays(s, num_ray, ray_org, ray_dir, m, o, cs, status_ptr());
@@ -924,7 +924,7 @@ int dm_batch_pix2tri_by_raycast(uint64_t stream_ptr, uint32_t num_mesh, const ui
   if (int e = sc.acquire(scratch, scratch_bytes, dm::cast_scratch_bytes(n, max_tri_per_mesh), s, nullptr)) return e;
   dm::CastScratch cs;
   dm::cast_scratch_carve(sc.ptr, n, max_tri_per_mesh, &cs);
-  DM_CUDA(cudaMemsetAsync(cs.counters, 0, 16, s));
+  DM_CUDA(cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, s));
   dm::CastOut o{pix2tri, pix2t, nullptr};
   dm::launch_batch_cast_pixels(s, dm::Segments{num_mesh, mesh2tri, mesh2vtx}, max_tri_per_mesh, tri2vtx, vtx2xyz,
                                bvhnodes, bvhnode2aabb, img_w, img_h, transforms_ndc2world, o, cs, status_ptr());

@@ -239,7 +239,7 @@ struct Tuning {
   uint32_t cast_leaf_min = kDefaultPhaseMin;
   uint32_t cast_ascend_min = kDefaultPhaseMin;
   // node entries after which the persistent cast, once a warp has no more
-  // rays to take, hands a ray entering a long chain to the warp tier
+  // rays to take, hands a ray entering a long chain to the team tier
   uint32_t cast_long_steps = kDefaultLongSteps;
   // batched build: 0 = every mesh sorted and linked on chip when the largest
   // fits (<= kSegMaxTri triangles), 1 = the global 64-bit sort
@@ -301,8 +301,10 @@ struct CastOut {
   float* hit_bc;      // optional, 3 per ray (1-u-v, u, v)
 };
 
+constexpr size_t kCastCounterBytes = 32;
+
 struct CastScratch {
-  uint32_t* counters;  // 4 words, zero on entry: work counter, two overflow counts
+  uint32_t* counters;  // kCastCounterBytes, zero on entry (see cast_job)
   uint32_t* list1;     // num_ray words
   uint32_t* list2;     // num_ray words
   void* pool;          // >= 16 * max(num_tri, 4096) bytes

@@ -174,7 +174,7 @@ enum LaneState : int {
 };
 
 // Chain links: branch j whose left child is leaf j and right child branch
-// j + 1 (runs of equal Morton codes build long runs of them).  The warp tier
+// j + 1 (runs of equal Morton codes build long runs of them).  The team tier
 // folds runs of at least kFoldMin links instead of walking them.
 constexpr uint32_t kFoldMin = 8;
 
@@ -291,7 +291,7 @@ __device__ __forceinline__ int phase_leaf(const MeshView& m, const Ray& r, Trav&
   return kLaneInner;
 }
 
-// A frame kind that only the warp tier pushes (see ChainFold); elsewhere none.
+// A frame kind that only the team tier pushes (see ChainFold); elsewhere none.
 struct NoFold {
   __device__ __forceinline__ int operator()(const uint4&, Trav&) const { return 0; }
 };
@@ -397,7 +397,7 @@ constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 // of the warp wait for it, or when nothing else can run.
 struct PhaseMins {
   uint32_t refill, leaf, ascend;
-  uint32_t long_steps;  // node entries after which a ray is handed to the warp tier
+  uint32_t long_steps;  // node entries after which a ray is handed to the team tier
 };
 
 // Persistent warps with per-lane ray refill, run in phases.  Each lane holds
@@ -413,7 +413,7 @@ struct PhaseMins {
 // Every lane still makes the same decisions in the same order, so results do
 // not depend on the thresholds.  Rays overflowing the on-chip stack, and
 // rays past mins.long_steps node entries at a long chain once the warp's
-// work is exhausted, go to ovf_list (their work index) for the warp tier.  kThreads threads per block and kStack on-chip frames per ray
+// work is exhausted, go to ovf_list (their work index) for the team tier.  kThreads threads per block and kStack on-chip frames per ray
 // are tuning choices (Tuning); the register bound (64 registers) keeps 2048
 // resident threads per SM.
 template <typename Job, int kThreads, int kStack>
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_pers
     }
     // Once the warp has no more rays to take, a ray past the step budget
     // that is about to enter a long chain would hold the kernel's end: it is
-    // handed to the warp tier, which folds chains 32 links at a time.
+    // handed to the team tier, which folds chains many links at a time.
     if (exhausted && state == kLaneInner && s.steps > mins.long_steps && long_chain_at(m, s.node, s.left, s.right))
       state = kLaneOverflow;
     if (state == kLaneDone) {
@@ -546,44 +546,90 @@ __global__ void __launch_bounds__(kCastThreads) k_cast_deep(Job job, const uint3
   if (bad) raise_status(status, kStatusBadIndex);
 }
 
-// ------------------------------------------------------------ warp tier
+// ------------------------------------------------------------ team tier
 // Rays that overflowed the persistent cast's stack, or that were about to
 // enter a long chain past its step budget once their warp had no more rays to
-// take, one warp each.  Every lane runs the same serial traversal on the
-// same state (the same loads, the same decisions), except at a chain: a run
-// of links, branches j whose left child is leaf j and right child branch
-// j + 1 (runs of equal Morton codes build them).  The recursion's result over
-// a chain c0..c1 is a fold from its far end: with x = F(c1 + 1), for j = c1
+// take, one team of warps each.  Every lane of a team runs the same serial
+// traversal on the same state (the same loads, the same decisions), except at a
+// chain: a run of links, branches j whose left child is leaf j and right child
+// branch j + 1 (runs of equal Morton codes build them).  The recursion's result
+// over a chain c0..c1 is a fold from its far end: with x = F(c1 + 1), for j = c1
 // down to c0
 //   x <- g_j(x):  neither child box hit: none;  only leaf j's box: h_j (its hit);
 //                 only branch j+1's box: x;  both, the leaf nearer: h_j if h_j
 //                 is a hit before branch j+1's entry, else pick(h_j, x);  both,
 //                 the branch nearer: x if x is a hit before leaf j's entry,
 //                 else pick(x, h_j)
-// (the rules of phase_inner / phase_leaf / phase_ascend).  So the warp pushes
+// (the rules of phase_inner / phase_leaf / phase_ascend).  So the team pushes
 // a fold frame, searches the tail c1 + 1 on its own, and on popping the frame
-// tests 32 * kFoldBatch links per round (kFoldBatch per lane) and folds them
-// with shuffles.
+// tests kFoldLinks links per warp and round, all loads in flight together, and
+// applies those that change the result in order.  Most change nothing: a link
+// whose branch box is hit and whose leaf holds no hit leaves x as it is.
 // On the duplicate-heavy soup 96% of the long rays' node entries are links.
+//
+// The kernel ends with its longest ray (26,600 links in 17 chains and 100 other
+// steps, of 1,048,576 rays in a soup of 4,194,304 triangles), and a round is a
+// few dependent trips to DRAM whatever it holds, so what counts is the number
+// of rounds.  That soup's cast, three draws: 2.1-3.3 ms with a warp per ray, 32
+// links per round and every link shuffled through; 1.06 ms with 128 links and
+// only the links that matter; 0.54-0.68 ms with teams of 4 warps that take their
+// rays from a counter (0.59-0.69 ms with fixed shares; teams of 8 warps
+// 0.71-0.84 ms and of 16 1.08-1.23 ms, fewer of which are resident).  2 links
+// per lane or 4 to 16 prefetched groups give the same within 3%.
 constexpr uint32_t kWarpAll = 0xffffffffu;
+constexpr uint32_t kTeamThreads = 128;
+constexpr uint32_t kTeamWarps = kTeamThreads / 32;
+constexpr uint32_t kFoldBatch = 4;  // links per lane and round
+constexpr uint32_t kFoldLinks = 32 * kFoldBatch;
 
-// The last link of the chain starting at link c0 (the same in every lane),
-// 256 records per round (8 per lane: 2.19 ms soup cast, 4 per lane 2.22,
-// 1 per lane 2.45).
-__device__ __forceinline__ uint32_t chain_last(const MeshView& m, uint32_t c0, uint32_t lane) {
+// A warp's part of a round: the leaves to test and their hits, then the links
+// to apply.  Two of the latter, so that a round does not wait for the team to
+// finish the one before.
+struct FoldShared {
+  float t[kFoldLinks];
+  uint32_t id[kFoldLinks];
+  uint8_t todo[kFoldLinks];
+  struct Op {
+    float t, enter;
+    uint32_t id, flags;
+  } op[2][kFoldLinks];
+  uint32_t num_op[2];
+  uint32_t cut[2];    // the first link to apply does not look at x
+  uint32_t first[2];  // chain_last: the first record of the warp's that is no link
+};
+
+// The warps that cast one ray together: the whole block, or a warp alone.  The
+// two sides of FoldShared are used in turn over all chains of the kernel, so
+// that a warp writes a side again only after a meeting of the team that the
+// others reach when they have read it.
+struct Team {
+  FoldShared* sh;  // the team's first warp's
+  uint32_t rank, warps, lane;
+  mutable uint32_t scan_side, fold_side;
+  __device__ __forceinline__ void sync() const {
+    if (warps > 1) __syncthreads();
+    else __syncwarp();
+  }
+};
+
+// The last link of the chain starting at link c0 (the same in every lane of the
+// team), 256 records per warp and round (8 per lane).
+__device__ __forceinline__ uint32_t chain_last(const MeshView& m, uint32_t c0, const Team& tm) {
   const uint32_t num_branch = m.num_tri - 1;
   uint32_t last = c0;
   for (;;) {
-    // lane l checks links last + 1 + 8 l .. last + 8 l + 8
+    const uint32_t side = tm.scan_side;
+    tm.scan_side ^= 1u;
+    // lane l of warp w checks links last + 1 + 256 w + 8 l and the 7 after it
+    const uint32_t base = last + 1 + 256 * tm.rank + 8 * tm.lane;
     bool ok[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const uint32_t j = last + 1 + 8 * lane + q;
       ok[q] = false;
-      if (j < num_branch) {
+      if (base + q < num_branch) {
         uint32_t l, r;
-        load_record(m.bvhnodes, j, l, r);
-        ok[q] = is_link(m, j, l, r);
+        load_record(m.bvhnodes, base + q, l, r);
+        ok[q] = is_link(m, base + q, l, r);
       }
     }
     uint32_t first_bad = 8;
@@ -591,62 +637,98 @@ __device__ __forceinline__ uint32_t chain_last(const MeshView& m, uint32_t c0, u
     for (int q = 7; q >= 0; --q)
       if (!ok[q]) first_bad = q;
     const uint32_t fail = __ballot_sync(kWarpAll, first_bad < 8);
+    uint32_t mine = 256;  // links of this warp's before the first other record
     if (fail != 0u) {
       const uint32_t l0 = static_cast<uint32_t>(__ffs(fail)) - 1u;
-      const uint32_t fb = __shfl_sync(kWarpAll, first_bad, l0);
-      return last + 8 * l0 + fb;
+      mine = 8 * l0 + __shfl_sync(kWarpAll, first_bad, l0);
     }
-    last += 256;
+    if (tm.warps == 1) {
+      if (mine < 256) return last + mine;
+    } else {
+      if (tm.lane == 0) tm.sh[tm.rank].first[side] = mine;
+      __syncthreads();
+      for (uint32_t w = 0; w < tm.warps; ++w) {
+        const uint32_t f = tm.sh[w].first[side];
+        if (f < 256) return last + 256 * w + f;
+      }
+    }
+    last += 256 * tm.warps;
   }
 }
 
-// Folds links hi, hi - 1, .., lo (at most 32 * kFoldBatch) into x.  Lane k
-// tests links hi - k - 32 q (q < kFoldBatch), all loads in flight together;
-// the warp then applies them in order, four shuffles per link.  One batch
-// per round measured fastest on the soup's cast (2.41 ms; 2 and 4 batches:
-// 2.62 and 2.61 ms).
-constexpr uint32_t kFoldBatch = 1;
-__device__ __forceinline__ Hit fold_links(const MeshView& m, const Ray& r, uint32_t lo, uint32_t hi, Hit x,
-                                          uint32_t lane, bool& bad) {
-  const uint32_t n = hi - lo + 1;
+// This warp's n links hi, hi - 1, .. (1 to kFoldLinks of them): tests them and
+// leaves those to be applied, in order, in sh.op[side].
+__device__ __forceinline__ void test_links(const MeshView& m, const Ray& r, uint32_t hi, uint32_t n, uint32_t lane,
+                                           FoldShared& sh, uint32_t side, bool& bad) {
+  const uint32_t lt = (1u << lane) - 1u;
   uint32_t flags[kFoldBatch];  // 1: leaf box hit, 2: branch box hit, 4: the leaf is the near child
   float far_enter[kFoldBatch];
-  Hit h[kFoldBatch];
+  uint32_t ntodo = 0;
 #pragma unroll
   for (uint32_t q = 0; q < kFoldBatch; ++q) {
-    flags[q] = 0;
-    far_enter[q] = 0.f;
-    h[q] = Hit{INFINITY, kUMax};
-    const uint32_t i = lane + 32 * q;
-    if (i < n) {
-      const uint32_t j = hi - i, leaf = m.num_tri - 1 + j;
-      float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
-      const bool ha = node_slab(m, r, leaf, a0, a1);
-      const bool hb = node_slab(m, r, j + 1, b0, b1);
-      const bool near_leaf = (ha && hb) ? tuple_lt(a0, a1, b0, b1) : ha;
-      flags[q] = (ha ? 1u : 0u) | (hb ? 2u : 0u) | (near_leaf ? 4u : 0u);
-      far_enter[q] = near_leaf ? b0 : a0;
-      if (ha) {
-        const uint32_t tri = __ldg(m.bvhnodes + static_cast<size_t>(leaf) * 3 + 1);
-        float t, u, v;
-        if (leaf_hit(m, r, tri, t, u, v, bad)) h[q] = Hit{t, tri};
-      }
-    }
+    // past the last link, that one is tested again and ignored
+    const uint32_t i = lane + 32 * q, j = hi - (i < n ? i : n - 1);
+    float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+    const bool ha = node_slab(m, r, m.num_tri - 1 + j, a0, a1);
+    const bool hb = node_slab(m, r, j + 1, b0, b1);
+    const bool near_leaf = (ha && hb) ? tuple_lt(a0, a1, b0, b1) : ha;
+    flags[q] = (ha ? 1u : 0u) | (hb ? 2u : 0u) | (near_leaf ? 4u : 0u);
+    far_enter[q] = near_leaf ? b0 : a0;
   }
 #pragma unroll
   for (uint32_t q = 0; q < kFoldBatch; ++q) {
-    for (uint32_t k = 0; k < 32 && 32 * q + k < n; ++k) {
-      const uint32_t f = __shfl_sync(kWarpAll, flags[q], k);
-      const float fe = __shfl_sync(kWarpAll, far_enter[q], k);
-      const Hit kh{__shfl_sync(kWarpAll, h[q].t, k), __shfl_sync(kWarpAll, h[q].id, k)};
-      if ((f & 3u) == 0u) {
-        x = Hit{INFINITY, kUMax};
-      } else if ((f & 3u) == 1u) {
-        x = kh;
-      } else if ((f & 3u) == 3u) {
-        if (f & 4u) x = (kh.id != kUMax && fe > kh.t) ? kh : pick(kh, x);
-        else x = (x.id != kUMax && fe > x.t) ? x : pick(x, kh);
-      }
+    const uint32_t i = lane + 32 * q;
+    const bool test = i < n && (flags[q] & 1u);
+    const uint32_t mask = __ballot_sync(kWarpAll, test);
+    if (test) sh.todo[ntodo + __popc(mask & lt)] = static_cast<uint8_t>(i);
+    ntodo += __popc(mask);
+  }
+  __syncwarp();
+  for (uint32_t c = lane; c < ntodo; c += 32) {
+    const uint32_t i = sh.todo[c], leaf = m.num_tri - 1 + (hi - i);
+    const uint32_t tri = __ldg(m.bvhnodes + static_cast<size_t>(leaf) * 3 + 1);
+    float t, u, v;
+    const bool h = leaf_hit(m, r, tri, t, u, v, bad);
+    sh.t[i] = h ? t : INFINITY;
+    sh.id[i] = h ? tri : kUMax;
+  }
+  __syncwarp();
+  uint32_t num = 0, has_cut = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kFoldBatch; ++q) {
+    const uint32_t i = lane + 32 * q;
+    Hit h{INFINITY, kUMax};
+    if (i < n && (flags[q] & 1u)) h = Hit{sh.t[i], sh.id[i]};
+    const uint32_t cut = __ballot_sync(kWarpAll, i < n && !(flags[q] & 2u));  // links that do not look at x
+    uint32_t todo = __ballot_sync(kWarpAll, i < n && (flags[q] & 2u) && h.id != kUMax) | cut;
+    if (cut != 0u) {  // what comes before the last of them is lost
+      todo &= 0xffffffffu << (31 - __clz(cut));
+      num = 0;
+      has_cut = 1;
+    }
+    if (todo >> lane & 1u)
+      sh.op[side][num + __popc(todo & lt)] = FoldShared::Op{h.t, far_enter[q], h.id, flags[q]};
+    num += __popc(todo);
+  }
+  if (lane == 0) {
+    sh.num_op[side] = num;
+    sh.cut[side] = has_cut;
+  }
+}
+
+// The links of a round applied to x, the warps' parts from the far end on.
+__device__ __forceinline__ Hit apply_links(const Team& tm, uint32_t side, Hit x) {
+  uint32_t w0 = 0;
+  for (uint32_t w = 1; w < tm.warps; ++w)
+    if (tm.sh[w].cut[side]) w0 = w;
+  for (uint32_t w = w0; w < tm.warps; ++w) {
+    const uint32_t num = tm.sh[w].num_op[side];
+    for (uint32_t k = 0; k < num; ++k) {
+      const FoldShared::Op o = tm.sh[w].op[side][k];
+      const Hit h{o.t, o.id};
+      if ((o.flags & 2u) == 0u) x = h;  // the leaf's hit, or none
+      else if (o.flags & 4u) x = o.enter > h.t ? h : pick(h, x);
+      else x = (x.id != kUMax && o.enter > x.t) ? x : pick(x, h);
     }
   }
   return x;
@@ -656,10 +738,10 @@ __device__ __forceinline__ Hit fold_links(const MeshView& m, const Ray& r, uint3
 // links pushes a fold frame {c0 | bit, c1 | bit, saved} and searches the
 // chain's tail (if its box is hit) with a fresh result.
 template <typename StackT>
-__device__ __forceinline__ int phase_inner_warp(const MeshView& m, const Ray& r, StackT stack, uint32_t cap, Trav& s,
-                                                bool& bad, uint32_t lane) {
+__device__ __forceinline__ int phase_inner_team(const MeshView& m, const Ray& r, StackT stack, uint32_t cap, Trav& s,
+                                                bool& bad, const Team& tm) {
   if (s.right != kUMax && is_link(m, s.node, s.left, s.right)) {
-    const uint32_t c0 = s.node, c1 = chain_last(m, c0, lane);
+    const uint32_t c0 = s.node, c1 = chain_last(m, c0, tm);
     if (c1 - c0 + 1 >= kFoldMin) {
       s.steps += 2 * (c1 - c0 + 1);  // its branches and leaves
       if (s.steps > 2 * m.num_tri) {
@@ -681,38 +763,47 @@ __device__ __forceinline__ int phase_inner_warp(const MeshView& m, const Ray& r,
   return phase_inner(m, r, stack, cap, s, bad);
 }
 
-constexpr uint32_t kChainPrefetch = 2;  // chunks of links prefetched ahead of the fold
+constexpr uint32_t kChainPrefetch = 8;  // groups of 32 links per warp prefetched ahead of the fold
 
 // Fold frames {c0 | bit, c1 | bit, saved}: the tail's result (the current
 // one) is folded through the chain, and the chain's result into `saved`.
 struct ChainFold {
   const MeshView& m;
   const Ray& r;
-  uint32_t lane;
+  const Team& tm;
   bool* bad;
   __device__ __forceinline__ int operator()(const uint4& f, Trav& s) const {
     if (!((f.x & kChainBit) && (f.y & kChainBit))) return 0;
     const uint32_t c0 = f.x & ~kChainBit, c1 = f.y & ~kChainBit;
     if (c0 > c1 || c1 + 1 >= 2 * m.num_tri - 1) return 2;
     Hit x = s.best;
-    const uint32_t nb = m.num_tri - 1;
-    for (uint32_t hi = c1;;) {
-      const uint32_t lo = hi - c0 >= 32 * kFoldBatch - 1 ? hi - (32 * kFoldBatch - 1) : c0;
-      // the links of the next kChainPrefetch chunks (lane k: one link each)
-      // toward L2 while this chunk is folded: a long chain's tree does not
-      // fit L2, and each chunk is otherwise a few dependent DRAM round trips
+    const uint32_t nb = m.num_tri - 1, total = c1 - c0 + 1, round = kFoldLinks * tm.warps;
+    for (uint32_t done = 0; done < total; done += round) {
+      const uint32_t side = tm.fold_side;
+      tm.fold_side ^= 1u;
+      // the warp's links of the next rounds (lane k: one link of each group)
+      // toward L2 while this round's are tested: a long chain's tree does not
+      // fit L2
 #pragma unroll
       for (uint32_t d = 0; d < kChainPrefetch; ++d) {
-        const int64_t j = static_cast<int64_t>(lo) - 1 - lane - 32 * static_cast<int64_t>(d);
-        if (j >= static_cast<int64_t>(c0)) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(m.bvhnodes + 3 * (nb + static_cast<uint64_t>(j))));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(m.aabb + 6 * (nb + static_cast<uint64_t>(j))));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(m.aabb + 6 * (static_cast<uint64_t>(j) + 1)));
+        const uint32_t i = done + (1 + d / kFoldBatch) * round + tm.rank * kFoldLinks + 32 * (d % kFoldBatch) + tm.lane;
+        if (i < total) {
+          const uint64_t j = c1 - i;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(m.bvhnodes + 3 * (nb + j)));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(m.aabb + 6 * (nb + j)));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(m.aabb + 6 * (j + 1)));
         }
       }
-      x = fold_links(m, r, lo, hi, x, lane, *bad);
-      if (lo == c0) break;
-      hi = lo - 1;
+      const uint32_t from = done + tm.rank * kFoldLinks;
+      if (from < total) {
+        test_links(m, r, c1 - from, total - from < kFoldLinks ? total - from : kFoldLinks, tm.lane, tm.sh[tm.rank],
+                   side, *bad);
+      } else if (tm.lane == 0) {
+        tm.sh[tm.rank].num_op[side] = 0;
+        tm.sh[tm.rank].cut[side] = 0;
+      }
+      tm.sync();
+      x = apply_links(tm, side, x);
     }
     --s.sp;
     s.best = pick(Hit{__uint_as_float(f.z), f.w}, x);
@@ -721,39 +812,58 @@ struct ChainFold {
 };
 
 template <typename StackT>
-__device__ __forceinline__ int trav_step_warp(const MeshView& m, const Ray& r, StackT stack, uint32_t cap, Trav& s,
-                                              bool& bad, uint32_t lane) {
-  int st = phase_inner_warp(m, r, stack, cap, s, bad, lane);
+__device__ __forceinline__ int trav_step_team(const MeshView& m, const Ray& r, StackT stack, uint32_t cap, Trav& s,
+                                              bool& bad, const Team& tm) {
+  int st = phase_inner_team(m, r, stack, cap, s, bad, tm);
   if (st == kLaneLeaf) st = phase_leaf(m, r, s, bad);
-  if (st == kLaneAscend) st = phase_ascend(m, r, stack, s, bad, ChainFold{m, r, lane, &bad});
+  if (st == kLaneAscend) st = phase_ascend(m, r, stack, s, bad, ChainFold{m, r, tm, &bad});
   return st == kLaneInner ? kStepContinue : (st == kLaneOverflow ? kStepOverflow : kStepDone);
 }
 
-// One warp per ray of list_in; a ray whose frames outgrow the warp's slice of
-// the pool goes to list_out.  Every lane keeps the same stack (the ring in its
-// own local memory, the spilled frames at the same addresses of the slice).
+// One team per ray of list_in; a ray whose frames outgrow a warp's slice of the
+// pool goes to list_out.  Every lane keeps the same stack (the ring in its own
+// local memory, the spilled frames at the same addresses of its warp's slice).
+// A team is a whole block while the rays are few, kTeamRays per block or
+// fewer: then the longest ray sets the kernel's end.  With more, their number
+// does, and each warp takes rays of its own.
+constexpr uint32_t kTeamRays = 8;
 template <typename Job>
-__global__ void __launch_bounds__(kCastThreads, 4) k_cast_warp(Job job, const uint32_t* list_in, const uint32_t* count_in,
-                                                           uint32_t* list_out, uint32_t* count_out, uint4* pool,
-                                                           uint64_t pool_frames, uint32_t max_tri, uint32_t* status) {
+__global__ void __launch_bounds__(kTeamThreads, 4) k_cast_team(Job job, const uint32_t* list_in, const uint32_t* count_in,
+                                                          uint32_t* take,
+                                                          uint32_t* list_out, uint32_t* count_out, uint4* pool,
+                                                          uint64_t pool_frames, uint32_t max_tri, uint32_t* status) {
   __shared__ float smem[64];
+  __shared__ FoldShared sh[kTeamWarps];
+  __shared__ uint32_t sh_take;
   job.prepare(smem);
   pdl_wait();
   pdl_launch_dependents();
   __syncthreads();
   const uint32_t num = *count_in;
   if (num == 0) return;
-  constexpr uint32_t kWarps = kCastThreads / 32;
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warps = static_cast<uint64_t>(gridDim.x) * kWarps;
-  const uint64_t wid = static_cast<uint64_t>(blockIdx.x) * kWarps + threadIdx.x / 32;
+  const uint32_t warp = threadIdx.x / 32;
+  const uint64_t warps = static_cast<uint64_t>(gridDim.x) * kTeamWarps;
+  const uint64_t wid = static_cast<uint64_t>(blockIdx.x) * kTeamWarps + warp;
+  const bool whole = num <= kTeamRays * gridDim.x;
+  const Team tm{whole ? sh : sh + warp, whole ? warp : 0u, whole ? kTeamWarps : 1u, threadIdx.x & 31u, 0u, 0u};
   uint64_t cap = pool_frames / warps;
   if (cap > 2ull * max_tri) cap = 2ull * max_tri;
   uint4 ring[kDeepRing];
   uint32_t lo = 0;
   const RingStack<kDeepRing> st{ring, pool + wid * cap, &lo};
   bool bad = false;
-  for (uint64_t k = wid; k < num; k += warps) {
+  for (;;) {
+    uint32_t k = 0;
+    if (tm.lane == 0 && tm.rank == 0) k = atomicAdd(take, 1u);
+    if (whole) {
+      if (threadIdx.x == 0) sh_take = k;
+      __syncthreads();
+      k = sh_take;
+      __syncthreads();
+    } else {
+      k = __shfl_sync(kWarpAll, k, 0);
+    }
+    if (k >= num) break;
     lo = 0;
     const uint32_t w = list_in[k];
     MeshView m{};
@@ -764,10 +874,10 @@ __global__ void __launch_bounds__(kCastThreads, 4) k_cast_warp(Job job, const ui
     int rc = kStepDone;
     if (trav_begin(m, r, s)) {
       do {
-        rc = trav_step_warp(m, r, st, static_cast<uint32_t>(cap), s, bad, lane);
+        rc = trav_step_team(m, r, st, static_cast<uint32_t>(cap), s, bad, tm);
       } while (rc == kStepContinue);
     }
-    if (lane == 0) {
+    if (tm.rank == 0 && tm.lane == 0) {
       if (rc == kStepDone) job.write(out, m, r, s.best);
       else list_out[atomicAdd(count_out, 1u)] = w;
     }
@@ -804,11 +914,11 @@ inline void launch_persistent(cudaStream_t s, const Job& job, const CastScratch&
 }
 
 // The tiered cast of every work index of `job`: the persistent cast; the
-// warp tier for the rays it hands over; for the rare ray whose frames outgrow
+// team tier for the rays it hands over; for the rare ray whose frames outgrow
 // a warp's slice, the serial tier with the pool split over those rays, then
-// with unbounded frames.  sc.counters (4 words) must be zero on entry: [0]
-// work counter, [1..3] the hand-over counts of tiers 1..3 (lists list1,
-// list2, list1 again).  The first tier's block size and on-chip stack depth
+// with unbounded frames.  sc.counters (kCastCounterBytes) must be zero on
+// entry: [0] work counter, [1..3] the hand-over counts of tiers 1..3 (lists
+// list1, list2, list1 again), [4] rays taken by the team tier.  The first tier's block size and on-chip stack depth
 // come from the current Tuning (kCastVariants lists the choices).
 template <typename Job>
 inline void cast_job(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, uint32_t* status) {
@@ -822,8 +932,8 @@ inline void cast_job(cudaStream_t s, const Job& job, const CastScratch& sc, uint
   const uint64_t pool_frames = sc.pool_bytes / kFrameBytes;
   uint4* pool = static_cast<uint4*>(sc.pool);
   const uint32_t deep_grid = 152 * 4;
-  launch_pdl(k_cast_warp<Job>, dim3(deep_grid), dim3(kCastThreads), 0, s, job, sc.list1, sc.counters + 1, sc.list2,
-             sc.counters + 2, pool, pool_frames, max_tri, status);
+  launch_pdl(k_cast_team<Job>, dim3(deep_grid), dim3(kTeamThreads), 0, s, job, sc.list1, sc.counters + 1,
+             sc.counters + 4, sc.list2, sc.counters + 2, pool, pool_frames, max_tri, status);
   launch_pdl(k_cast_deep<Job>, dim3(deep_grid), dim3(kCastThreads), 0, s, job, sc.list2, sc.counters + 2, sc.list1,
              sc.counters + 3, pool, pool_frames, 0u, max_tri, status);
   const uint32_t cap3 = max_tri < 2 ? 2u : max_tri;

@@ -228,7 +228,7 @@ int cast_request(cudaStream_t st, const HostMesh& hm, const DevMesh& m, const dm
   CastScratch cs;
   const uint32_t n = (r.kind == DM_REQ_CAST_RAYS) ? r.num_ray : r.img_w * r.img_h;
   cast_scratch_carve(sl.cast_scratch, n, hm.T, &cs);
-  if (cudaMemsetAsync(cs.counters, 0, 16, st) != cudaSuccess) return DM_ERR_CUDA;
+  if (cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, st) != cudaSuccess) return DM_ERR_CUDA;
   CastOut o{sl.d_hit, sl.d_t, nullptr};
   if (r.kind == DM_REQ_CAST_RAYS) {
     float* org = sl.d_rays;
