@@ -696,6 +696,19 @@ struct BatchJob {
     return true;
   }
 
+  template <typename T>
+  __device__ __forceinline__ static const T* lane_ptr(const T* p, int from) {
+    return reinterpret_cast<const T*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(p), from));
+  }
+  __device__ __forceinline__ void share(MeshView& mv, int from) const {
+    mv.num_tri = __shfl_sync(0xffffffffu, mv.num_tri, from);
+    mv.num_vtx = __shfl_sync(0xffffffffu, mv.num_vtx, from);
+    mv.tri2vtx = lane_ptr(mv.tri2vtx, from);
+    mv.vtx2xyz = lane_ptr(mv.vtx2xyz, from);
+    mv.bvhnodes = lane_ptr(mv.bvhnodes, from);
+    mv.aabb = lane_ptr(mv.aabb, from);
+  }
+
   __device__ __forceinline__ void write(uint32_t out, const MeshView&, const Ray&, const Hit& h) const {
     o.hit_tri[out] = h.id;
     if (o.hit_t) o.hit_t[out] = h.t;

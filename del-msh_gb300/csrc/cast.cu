@@ -47,6 +47,8 @@ struct SingleJob {
     return true;
   }
 
+  __device__ __forceinline__ void share(MeshView& mv, int) const { mv = m; }
+
   __device__ __forceinline__ void write(uint32_t out, const MeshView& mv, const Ray& r, const Hit& h) const {
     o.hit_tri[out] = h.id;
     if (o.hit_t) o.hit_t[out] = h.t;
@@ -86,7 +88,7 @@ void cast_scratch_carve(void* base, uint32_t num_ray, uint32_t num_tri, CastScra
 }
 
 void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const float* t_ndc2world, const MeshView& m,
-                        const CastOut& o, const CastScratch& sc, uint32_t* status) {
+                        const CastOut& o, const CastScratch& sc, uint32_t* status, bool busy) {
   SingleJob job{};
   job.m = m;
   job.img_w = img_w;
@@ -101,18 +103,18 @@ void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const fl
   job.num_work = job.tiles_x * tiles_y * 32u;
   job.t_ndc2world = t_ndc2world;
   job.o = o;
-  cast_job(s, job, sc, m.num_tri, status);
+  cast_job(s, job, sc, m.num_tri, status, busy);
 }
 
 void launch_cast_rays(cudaStream_t s, uint32_t num_ray, const float* ray_org, const float* ray_dir,
-                      const MeshView& m, const CastOut& o, const CastScratch& sc, uint32_t* status) {
+                      const MeshView& m, const CastOut& o, const CastScratch& sc, uint32_t* status, bool busy) {
   SingleJob job{};
   job.m = m;
   job.num_work = num_ray;
   job.ray_org = ray_org;
   job.ray_dir = ray_dir;
   job.o = o;
-  cast_job(s, job, sc, m.num_tri, status);
+  cast_job(s, job, sc, m.num_tri, status, busy);
 }
 
 }  // namespace dm

@@ -315,10 +315,12 @@ size_t cast_scratch_bytes(uint32_t num_ray, uint32_t num_tri);
 void cast_scratch_carve(void* base, uint32_t num_ray, uint32_t num_tri, CastScratch* out);
 
 // Pixels of an img_w x img_h image (ray_for_pixel.h) or explicit rays.
+// busy: the GPU has other work beside this cast (see launch_tiers)
 void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const float* t_ndc2world, const MeshView& m,
-                        const CastOut& o, const CastScratch& sc, uint32_t* status);
+                        const CastOut& o, const CastScratch& sc, uint32_t* status, bool busy = false);
 void launch_cast_rays(cudaStream_t s, uint32_t num_ray, const float* ray_org, const float* ray_dir,
-                      const MeshView& m, const CastOut& o, const CastScratch& sc, uint32_t* status);
+                      const MeshView& m, const CastOut& o, const CastScratch& sc, uint32_t* status,
+                      bool busy = false);
 
 // img_w x img_h pixels per mesh of a batch, per-mesh ndc->world transforms
 // (16 floats each); output slot of pixel p of mesh m is m*img_w*img_h + p.

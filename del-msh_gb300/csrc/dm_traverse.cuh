@@ -36,15 +36,16 @@
 // finished takes the next ray index from a global counter (one atomic per
 // warp), so lanes stay busy while long rays finish, and the rarer phases
 // wait until several lanes need them (k_cast_persistent).  Frames live in a
-// kCastStack-entry on-chip (local) stack; a ray that needs more is appended to
-// an overflow list and re-cast from scratch by a second kernel whose per-ray
-// stacks are carved from a global pool (capacity chosen on the device from
-// the overflow count), and anything still deeper by a third kernel with
-// capacity num_tri, which no tree can exceed.  Those two keep the top 64
-// frames of each stack in an on-chip ring (RingStack) and only its bottom in
-// the pool.  Duplicate Morton codes produce
-// long chains (a run of k equal codes is a chain of height k), which is where
-// the deeper tiers are used.
+// kCastStack-entry on-chip (local) stack.  A second kernel (k_cast_tail) finishes
+// what the warps hand over: long rays, parked with their stacks and searched by
+// several lanes each (split tier); rays that overflowed the stack or are about to
+// enter a long chain, re-cast from scratch by teams of warps that fold chains
+// (team tier); and the rare ray whose frames outgrow a team's slice of the global
+// pool, re-cast with stacks carved from the whole pool, at last with capacity
+// num_tri, which no tree can exceed.  The latter two keep the top 64 frames of
+// each stack in an on-chip ring (RingStack) and only its bottom in the pool.
+// Duplicate Morton codes produce long chains (a run of k equal codes is a chain of
+// height k), which is where the team tier is used.
 #pragma once
 #include "dm_device.cuh"
 #include "dm_internal.h"
@@ -138,6 +139,7 @@ struct RingStack {
 };
 
 constexpr uint32_t kChainBit = 0x80000000u;  // frame.x flag of a chain frame (node ids are < 2^31)
+constexpr uint32_t kGivenBits = 0xC0000000u;  // frame.x of a given frame, with the lane that has it (links are < 2^30)
 
 // Per-ray traversal state between phases.
 struct Trav {
@@ -171,6 +173,9 @@ enum LaneState : int {
   kLaneAscend = 3,
   kLaneOverflow = 4,  // the on-chip stack is full: the ray is re-cast by a deeper tier
   kLaneDone = 5,      // s.best is the ray's result
+  kLaneJoin = 6,      // its next frame was given to another lane, whose result it needs
+  kLaneHelped = 7,    // a given frame's result is in s.best
+  kLaneParked = 8,    // waits to be parked for the split tier
 };
 
 // Chain links: branch j whose left child is leaf j and right child branch
@@ -223,17 +228,14 @@ __device__ __forceinline__ int phase_inner(const MeshView& m, const Ray& r, Stac
                                            bool& bad) {
   const uint32_t* __restrict__ bn = m.bvhnodes;
   const uint32_t num_node = 2 * m.num_tri - 1;
-  if (++s.steps > num_node + 1) {
-    bad = true;
-    return kLaneDone;
-  }
+  ++s.steps;
   if (s.right == kUMax) {
     s.leaf_tri = s.left;
     s.leaf_far = false;
     return kLaneLeaf;
   }
   const uint32_t node = s.node, left = s.left, right = s.right;
-  if (left >= num_node || right >= num_node) {
+  if (max(left, right) >= num_node || s.steps > num_node + 1) {
     bad = true;
     return kLaneDone;
   }
@@ -243,22 +245,13 @@ __device__ __forceinline__ int phase_inner(const MeshView& m, const Ray& r, Stac
   float l0 = 0.f, l1 = 0.f, r0 = 0.f, r1 = 0.f;
   const bool hl = node_slab(m, r, left, l0, l1);
   const bool hr = node_slab(m, r, right, r0, r1);
-  if (!hl && !hr) return kLaneAscend;
-  const bool near_left = (hl && hr) ? tuple_lt(l0, l1, r0, r1) : hl;
+  const bool both = hl && hr;
+  const bool near_left = both ? tuple_lt(l0, l1, r0, r1) : hl;
   const uint32_t nn = near_left ? left : right, nf = near_left ? right : left;
   const uint32_t n_l = near_left ? ll : rl, n_r = near_left ? lr : rr;
-  const bool has_far = hl && hr;
   const float far_enter = near_left ? r0 : l0;
-  if (n_r == kUMax) {  // near child is a leaf holding triangle n_l
-    s.leaf_tri = n_l;
-    s.leaf_far = has_far;
-    s.far_enter = far_enter;
-    s.node = nf;
-    s.left = near_left ? rl : ll;
-    s.right = near_left ? rr : lr;
-    return kLaneLeaf;
-  }
-  if (has_far) {
+  const bool near_leaf = n_r == kUMax;  // the near child is a leaf holding triangle n_l
+  if (both && !near_leaf) {
     const bool link = !near_left && left == m.num_tri - 1 + node && right == node + 1;
     if (link && node == s.chain_next && s.best.id == kUMax) {
       // extend the chain frame on top: its last link becomes `node`
@@ -266,19 +259,22 @@ __device__ __forceinline__ int phase_inner(const MeshView& m, const Ray& r, Stac
       stack.store(s.sp - 1, make_uint4(f.x, node, f.z, f.w));
     } else {
       if (s.sp >= cap) return kLaneOverflow;
-      if (link)
-        stack.store(s.sp++, make_uint4(kChainBit | node, node, __float_as_uint(s.best.t), s.best.id));
-      else
-        stack.store(s.sp++, make_uint4(nf, __float_as_uint(far_enter), __float_as_uint(s.best.t), s.best.id));
+      stack.store(s.sp++, make_uint4(link ? kChainBit | node : nf, link ? node : __float_as_uint(far_enter),
+                                     __float_as_uint(s.best.t), s.best.id));
     }
     s.chain_next = link ? node + 1 : kUMax;
     s.best = Hit{INFINITY, kUMax};
   }
-  // without a far child R(node) == R(near): no pending decision, no frame
-  s.node = nn;
-  s.left = n_l;
-  s.right = n_r;
-  return kLaneInner;
+  // without a far child R(node) == R(near): no pending decision, no frame.
+  // What the next phase does not read may be written all the same: the three
+  // outcomes then differ by selects and not by branches.
+  s.leaf_tri = n_l;
+  s.leaf_far = both;
+  s.far_enter = far_enter;
+  s.node = near_leaf ? nf : nn;
+  s.left = near_leaf ? (near_left ? rl : ll) : n_l;
+  s.right = near_leaf ? (near_left ? rr : lr) : n_r;
+  return hl || hr ? (near_leaf ? kLaneLeaf : kLaneInner) : kLaneAscend;
 }
 
 // The pending triangle test.  After a near leaf the far child is searched
@@ -298,13 +294,14 @@ struct NoFold {
 
 // Pops frames until a far child is to be searched (kLaneInner) or the stack
 // is empty (kLaneDone).  `fold` consumes the frames of its own kind (1), or
-// reports a malformed one (2).
+// reports a malformed one (2).  The `given` bottom frames are in the hands of
+// other lanes: once the others are popped the lane is at a join (kLaneJoin).
 template <typename StackT, typename Fold = NoFold>
 __device__ __forceinline__ int phase_ascend(const MeshView& m, const Ray& r, StackT stack, Trav& s, bool& bad,
-                                            const Fold& fold = Fold{}) {
+                                            const Fold& fold = Fold{}, uint32_t given = 0) {
   const uint32_t num_node = 2 * m.num_tri - 1;
   s.chain_next = kUMax;
-  while (s.sp > 0) {
+  while (s.sp > given) {
     const uint4 f = stack.load(s.sp - 1);
     const int folded = fold(f, s);
     if (folded == 1) continue;
@@ -352,7 +349,7 @@ __device__ __forceinline__ int phase_ascend(const MeshView& m, const Ray& r, Sta
       return kLaneInner;
     }
   }
-  return kLaneDone;
+  return given == 0 ? kLaneDone : kLaneJoin;
 }
 
 // One node entry and everything up to the next one (the phases back to
@@ -384,6 +381,9 @@ constexpr int kCastThreads = 128;
 // (2M-triangle torus 1920x1080 cast / 4096-mesh batched cast): 1 step 0.528 / 4.94 ms, 2 steps
 // 0.480 / 4.61, 3 steps 0.466 / 4.54, 4 steps 0.469 / 5.33, 6 steps 0.561 / 6.20.
 constexpr int kInnerSteps = 3;
+// Of the split tier's loop (2M torus 1920 x 1080 / 641 x 479 on a 66k torus, parked at 64 entries): 1 step 542 /
+// 153 us, 2 steps 514 / 154, 3 steps 513 / 156.
+constexpr int kTailSteps = 2;
 constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 
 // A Job maps a work index to (mesh, ray, output slot):
@@ -391,6 +391,8 @@ constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 //   __device__ void prepare(float* smem) const;    once per block, before __syncthreads
 //   __device__ bool fetch(uint32_t w, const float* smem, MeshView& m, Ray& r, uint32_t& out) const;
 //                                                   false: w is padding, nothing to do
+//   __device__ void share(MeshView& m, int from) const;
+//                                                   m becomes that of lane `from` (all lanes call it)
 //   __device__ void write(uint32_t out, const MeshView& m, const Ray& r, const Hit& h) const;
 
 // Thresholds of the phased loop: a phase runs when at least this many lanes
@@ -398,6 +400,14 @@ constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 struct PhaseMins {
   uint32_t refill, leaf, ascend;
   uint32_t long_steps;  // node entries after which a ray is handed to the team tier
+  uint32_t park_steps;  // node entries after which a ray is parked for the split tier
+  uint32_t share;       // rays a warp takes at a time, at most
+};
+
+struct Parked {
+  uint4* rays;  // per ray: {work, node, left, right}, {sp, steps, best}, the frames
+  uint32_t* count;
+  uint32_t capacity, stride;
 };
 
 // Persistent warps with per-lane ray refill, run in phases.  Each lane holds
@@ -407,20 +417,21 @@ struct PhaseMins {
 // the refill each happen about once per ray but in some lane nearly every
 // iteration, so running them whenever any lane needs one leaves most lanes
 // idle through them; waiting until `mins` lanes need one runs each for more
-// lanes at once, while the others go on entering nodes.  Once the warp's
-// refill finds no more work, a waiting lane would only lengthen the warp's
-// longest ray, so from then on every phase runs whenever a lane needs it.
-// Every lane still makes the same decisions in the same order, so results do
-// not depend on the thresholds.  Rays overflowing the on-chip stack, and
-// rays past mins.long_steps node entries at a long chain once the warp's
-// work is exhausted, go to ovf_list (their work index) for the team tier.  kThreads threads per block and kStack on-chip frames per ray
-// are tuning choices (Tuning); the register bound (64 registers) keeps 2048
-// resident threads per SM.
+// lanes at once, while the others go on entering nodes.  Every lane still makes
+// the same decisions in the same order, so results do not depend on the
+// thresholds.  Rays overflowing the on-chip stack, and rays past mins.long_steps
+// node entries at a long chain once the warp's work is exhausted, go to ovf_list
+// (their work index) for the team tier.  kThreads threads per block and kStack
+// on-chip frames per ray are tuning choices (Tuning); the register bound (64
+// registers) keeps 2048 resident threads per SM.  The loop after the work has run
+// out is a second copy of the phases: with one loop for both, the parking code
+// cost the first one 100 bytes of spills (batched cast 1.26 -> 1.48 ms).
 template <typename Job, int kThreads, int kStack>
 __global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_persistent(Job job, uint32_t* work_counter,
                                                                                  uint32_t* ovf_list,
                                                                                  uint32_t* ovf_count,
-                                                                                 uint32_t* status, PhaseMins mins) {
+                                                                                 uint32_t* status, PhaseMins mins,
+                                                                                 Parked parked) {
   __shared__ float smem[64];
   job.prepare(smem);
   __syncthreads();
@@ -439,12 +450,14 @@ __global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_pers
     // refill idle lanes with consecutive work indices
     const uint32_t idle = __ballot_sync(kAll, state == kLaneIdle);
     if (idle != 0u && !exhausted && (idle == kAll || static_cast<uint32_t>(__popc(idle)) >= mins.refill)) {
+      const uint32_t take = min(static_cast<uint32_t>(__popc(idle)), mins.share);
       uint32_t base = 0;
-      if (lane == static_cast<uint32_t>(__ffs(idle) - 1)) base = atomicAdd(work_counter, __popc(idle));
+      if (lane == static_cast<uint32_t>(__ffs(idle) - 1)) base = atomicAdd(work_counter, take);
       base = __shfl_sync(kAll, base, __ffs(idle) - 1);
-      if (base + __popc(idle) >= job.num_work) exhausted = true;  // warp-uniform: no work after this
-      if (state == kLaneIdle) {
-        const uint32_t w = base + __popc(idle & lt_mask);
+      if (base + take >= job.num_work) exhausted = true;  // warp-uniform: no work after this
+      const uint32_t rank = __popc(idle & lt_mask);
+      if (state == kLaneIdle && rank < take) {
+        const uint32_t w = base + rank;
         if (w < job.num_work && job.fetch(w, smem, m, r, out)) {
           work = w;
           if (trav_begin(m, r, s)) state = kLaneInner;
@@ -452,11 +465,8 @@ __global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_pers
         }
       }
     }
-    if (__all_sync(kAll, state == kLaneIdle)) {
-      if (exhausted) break;
-      continue;
-    }
-    const uint32_t leaf_min = exhausted ? 1u : mins.leaf, ascend_min = exhausted ? 1u : mins.ascend;
+    if (exhausted) break;
+    if (__all_sync(kAll, state == kLaneIdle)) continue;
     // Up to kInnerSteps node entries per iteration: the warp's votes and
     // phase decisions are paid once for several entries, and a lane that
     // leaves the inner phase early waits for the others' entries.
@@ -465,19 +475,14 @@ __global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_pers
       if (state == kLaneInner) state = phase_inner(m, r, stack, kStack, s, bad);
     uint32_t inner = __ballot_sync(kAll, state == kLaneInner);
     const uint32_t leaf = __ballot_sync(kAll, state == kLaneLeaf);
-    if (leaf != 0u && (inner == 0u || static_cast<uint32_t>(__popc(leaf)) >= leaf_min)) {
+    if (leaf != 0u && (inner == 0u || static_cast<uint32_t>(__popc(leaf)) >= mins.leaf)) {
       if (state == kLaneLeaf) state = phase_leaf(m, r, s, bad);
       inner = __ballot_sync(kAll, state == kLaneInner);
     }
     const uint32_t asc = __ballot_sync(kAll, state == kLaneAscend);
-    if (asc != 0u && (inner == 0u || static_cast<uint32_t>(__popc(asc)) >= ascend_min)) {
+    if (asc != 0u && (inner == 0u || static_cast<uint32_t>(__popc(asc)) >= mins.ascend)) {
       if (state == kLaneAscend) state = phase_ascend(m, r, stack, s, bad);
     }
-    // Once the warp has no more rays to take, a ray past the step budget
-    // that is about to enter a long chain would hold the kernel's end: it is
-    // handed to the team tier, which folds chains many links at a time.
-    if (exhausted && state == kLaneInner && s.steps > mins.long_steps && long_chain_at(m, s.node, s.left, s.right))
-      state = kLaneOverflow;
     if (state == kLaneDone) {
       job.write(out, m, r, s.best);
       state = kLaneIdle;
@@ -486,62 +491,44 @@ __global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_pers
       state = kLaneIdle;
     }
   }
-  if (bad) raise_status(status, kStatusBadIndex);
-}
-
-// Re-casts the work indices of list_in with stacks carved from the pool.
-// cap_fixed == 0 chooses the capacity from the number of rays to process.
-template <typename Job>
-__global__ void __launch_bounds__(kCastThreads) k_cast_deep(Job job, const uint32_t* list_in, const uint32_t* count_in,
-                                                           uint32_t* list_out, uint32_t* count_out, uint4* pool,
-                                                           uint64_t pool_frames, uint32_t cap_fixed,
-                                                           uint32_t max_tri, uint32_t* status) {
-  __shared__ float smem[64];
-  job.prepare(smem);
-  pdl_wait();
-  pdl_launch_dependents();
-  __syncthreads();
-  const uint32_t num = *count_in;
-  if (num == 0) return;
-  uint64_t cap = cap_fixed;
-  if (cap == 0) {
-    cap = pool_frames / num;
-    if (cap < 256) cap = 256;
-    const uint64_t cap_max = 2ull * max_tri;  // never more than the deepest possible tree needs
-    if (cap > cap_max) cap = cap_max;
-  }
-  if (cap > pool_frames) cap = pool_frames;
-  const uint64_t threads = static_cast<uint64_t>(gridDim.x) * kCastThreads;
-  uint64_t slots = pool_frames / cap;
-  if (slots > threads) slots = threads;
-  const uint64_t slot = static_cast<uint64_t>(threadIdx.x) * gridDim.x + blockIdx.x;  // spread over blocks
-  if (slot >= slots) return;
-  uint4 ring[kDeepRing];
-  uint32_t lo = 0;
-  const RingStack<kDeepRing> st{ring, pool + slot * cap, &lo};
-  bool bad = false;
-  for (uint64_t k = slot; k < num; k += slots) {
-    lo = 0;
-    const uint32_t w = list_in[k];
-    MeshView m{};
-    Ray r{};
-    uint32_t out = 0;
-    if (!job.fetch(w, smem, m, r, out)) continue;
-    Trav s{};
-    int rc = kStepDone;
-    if (trav_begin(m, r, s)) {
-      do {
-        rc = trav_step(m, r, st, static_cast<uint32_t>(cap), s, bad);
-      } while (rc == kStepContinue);
+  // The warp has no more rays to take: a waiting lane would only lengthen its
+  // longest ray, so every phase runs whenever a lane needs it.  A ray past the
+  // step budget that is about to enter a long chain would hold the kernel's end:
+  // it is handed to the team tier, which folds chains many links at a time.  One
+  // that goes on for long stops here and is parked for the split tier.
+  uint32_t park_steps = mins.park_steps;
+  for (;;) {
+    while (__any_sync(kAll, state == kLaneInner || state == kLaneLeaf || state == kLaneAscend)) {
+#pragma unroll
+      for (int k = 0; k < kInnerSteps; ++k)
+        if (state == kLaneInner) state = phase_inner(m, r, stack, kStack, s, bad);
+      if (state == kLaneLeaf) state = phase_leaf(m, r, s, bad);
+      if (state == kLaneAscend) state = phase_ascend(m, r, stack, s, bad);
+      if (state == kLaneInner && s.steps > mins.long_steps && long_chain_at(m, s.node, s.left, s.right))
+        state = kLaneOverflow;
+      if (state == kLaneInner && s.steps > park_steps) state = kLaneParked;
+      if (state == kLaneDone) {
+        job.write(out, m, r, s.best);
+        state = kLaneIdle;
+      } else if (state == kLaneOverflow) {
+        ovf_list[atomicAdd(ovf_count, 1u)] = work;
+        state = kLaneIdle;
+      }
     }
-    if (rc == kStepDone) {
-      job.write(out, m, r, s.best);
-    } else if (list_out) {
-      list_out[atomicAdd(count_out, 1u)] = w;
-    } else {
-      raise_status(status, kStatusStackOverflow);
-      job.write(out, m, r, Hit{INFINITY, kUMax});
+    if (!__any_sync(kAll, state == kLaneParked)) break;
+    if (state == kLaneParked) {
+      const uint32_t at = atomicAdd(parked.count, 1u);
+      if (at < parked.capacity) {
+        uint4* to = parked.rays + static_cast<size_t>(at) * parked.stride;
+        to[0] = make_uint4(work, s.node, s.left, s.right);
+        to[1] = make_uint4(s.sp, s.steps, __float_as_uint(s.best.t), s.best.id);
+        for (uint32_t k = 0; k < s.sp; ++k) to[2 + k] = frames[k];
+        state = kLaneIdle;
+      } else {
+        state = kLaneInner;  // no room: it goes on here
+      }
     }
+    park_steps = kUMax;
   }
   if (bad) raise_status(status, kStatusBadIndex);
 }
@@ -579,7 +566,7 @@ __global__ void __launch_bounds__(kCastThreads) k_cast_deep(Job job, const uint3
 constexpr uint32_t kWarpAll = 0xffffffffu;
 constexpr uint32_t kTeamThreads = 128;
 constexpr uint32_t kTeamWarps = kTeamThreads / 32;
-constexpr uint32_t kFoldBatch = 4;  // links per lane and round
+constexpr uint32_t kFoldBatch = 2;  // links per lane and round
 constexpr uint32_t kFoldLinks = 32 * kFoldBatch;
 
 // A warp's part of a round: the leaves to test and their hits, then the links
@@ -820,50 +807,228 @@ __device__ __forceinline__ int trav_step_team(const MeshView& m, const Ray& r, S
   return st == kLaneInner ? kStepContinue : (st == kLaneOverflow ? kStepOverflow : kStepDone);
 }
 
-// One team per ray of list_in; a ray whose frames outgrow a warp's slice of the
-// pool goes to list_out.  Every lane keeps the same stack (the ring in its own
-// local memory, the spilled frames at the same addresses of its warp's slice).
-// A team is a whole block while the rays are few, kTeamRays per block or
-// fewer: then the longest ray sets the kernel's end.  With more, their number
-// does, and each warp takes rays of its own.
-constexpr uint32_t kTeamRays = 8;
+// Rays that outlast the rest.  When the work runs out, a cast is as long as its
+// longest ray from there on, and long rays come in bundles: neighbouring pixels
+// graze the same silhouette, so one warp holds many and the others run empty.
+// The persistent cast therefore parks rays past park_steps node entries, stack
+// and all, and this kernel deals them out again, as few per warp as it can, and
+// lets the lanes that hold none help: F(n) of a frame's far child depends on
+// nothing outside n, so a lane may search it for another.  A lane gives away its
+// frames from the bottom, the largest subtrees first.  Popping a given frame, it
+// joins: it drops the helper if the recursion skips the far child (nearer result
+// than the far box), else it waits for the helper's result and picks it after
+// its own, which is what searching the far child would have done, as pick is
+// associative.  Results are therefore the same bits; only subtrees that are
+// skipped after all are searched in vain.
+// What bounds it: a node entry is about 1,250 cycles (two of them and a leaf test
+// or a pop per iteration), and the helpers' ramp.  Measured (cast alone, start ->
+// with parking, 3% of which are the branches saved in phase_inner): 2M torus
+// 1920 x 1080 (longest ray 504 entries) 613 -> 421 us; 512 x 512 of a deformed
+// 502k torus (338) 334 -> 237 us; 641 x 479 of a 66k torus (207) 198 -> 162 us;
+// 16,384 rays on a jittered 200k sphere (209) 195 -> 131 us.  Casts with no long
+// rays keep their time (4.2M rays on 1,024 small meshes, at most 100 entries:
+// 1.26 -> 1.23 ms).
+// A ray that runs into a long chain or out of stack is linked into the block's
+// own list (`handed`, by parked index; the next one in its second word) and cast
+// by the block as a team afterwards.
+template <typename Job, int kStack>
+__device__ __forceinline__ void cast_split(const Job& job, const float* smem, const Parked& parked, uint32_t num,
+                                           uint32_t* take, uint2* sh_deal, uint32_t* handed, uint32_t long_steps,
+                                           uint32_t* status) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t lt_mask = (1u << lane) - 1u;
+  const uint32_t warps = gridDim.x * (blockDim.x / 32);
+  const uint32_t share = min(32u, (num + warps - 1) / warps);  // rays per warp at a time
+  uint4 frames[kStack];
+  LocalStack stack{frames};
+  MeshView m{};
+  Ray r{};
+  Trav s{};
+  uint32_t out = 0, slot = kUMax;
+  int state = kLaneIdle;
+  bool bad = false;
+  uint32_t given = 0, parent = kUMax;  // frames given to other lanes; the lane this one helps
+  // Every iteration enters a node, tests a leaf, pops a frame or joins for some
+  // lane, and each happens at most once per node of a well-formed tree.
+  uint32_t rounds_left = 0;
+  for (;;) {
+    const uint32_t idle = __ballot_sync(kAll, state == kLaneIdle);
+    if (idle == kAll) {  // the next parked rays
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(take, share);
+      base = __shfl_sync(kAll, base, 0);
+      if (base >= num) break;
+      if (lane < share && base + lane < num) {
+        const uint4* from = parked.rays + static_cast<size_t>(base + lane) * parked.stride;
+        const uint4 a = from[0], b = from[1];
+        slot = base + lane;
+        if (job.fetch(a.x, smem, m, r, out)) {
+          s = Trav{};
+          s.node = a.y;
+          s.left = a.z;
+          s.right = a.w;
+          s.sp = b.x;
+          s.steps = b.y;
+          s.chain_next = kUMax;
+          s.best = Hit{__uint_as_float(b.z), b.w};
+          for (uint32_t k = 0; k < s.sp; ++k) frames[k] = from[2 + k];
+          parent = kUMax;
+          given = 0;
+          state = kLaneInner;
+        }
+      }
+      rounds_left = __reduce_max_sync(kAll, min(m.num_tri, 1u << 28)) * 8u + 1024u;
+      continue;
+    }
+    if (rounds_left-- == 0u) {
+      if (state != kLaneIdle && parent == kUMax) job.write(out, m, r, Hit{INFINITY, kUMax});
+      bad = true;
+      state = kLaneIdle;
+      continue;
+    }
+    if (idle != 0u) {
+      // lanes with a frame to give: the bottom one not yet given
+      uint32_t far = kUMax;
+      const bool busy = state == kLaneInner || state == kLaneLeaf || state == kLaneAscend;
+      if (busy && s.sp > given + (state == kLaneAscend ? 1u : 0u)) far = frames[given].x;
+      // in a malformed tree nothing is split, so that the step budget bounds all work
+      const uint32_t any_bad = __ballot_sync(kAll, bad);
+      const bool can = any_bad == 0u && !(far & kChainBit);
+      const uint32_t givers = __ballot_sync(kAll, can);
+      const uint32_t n = min(__popc(idle), __popc(givers));
+      if (n != 0u) {
+        const uint32_t rank_g = __popc(givers & lt_mask), rank_i = __popc(idle & lt_mask);
+        const bool gives = can && rank_g < n, takes = state == kLaneIdle && rank_i < n;
+        uint2* deal = sh_deal + (threadIdx.x & ~31u);
+        if (gives) deal[rank_g].x = lane;
+        if (takes) deal[rank_i].y = lane;
+        __syncwarp();
+        const uint32_t from = takes ? deal[rank_i].x : lane;
+        const uint32_t node = __shfl_sync(kAll, far, from);
+        r.org = make_float3(__shfl_sync(kAll, r.org.x, from), __shfl_sync(kAll, r.org.y, from),
+                            __shfl_sync(kAll, r.org.z, from));
+        r.dir = make_float3(__shfl_sync(kAll, r.dir.x, from), __shfl_sync(kAll, r.dir.y, from),
+                            __shfl_sync(kAll, r.dir.z, from));
+        r.inv = make_float3(__shfl_sync(kAll, r.inv.x, from), __shfl_sync(kAll, r.inv.y, from),
+                            __shfl_sync(kAll, r.inv.z, from));
+        r.nz = __shfl_sync(kAll, r.nz ? 1 : 0, from) != 0;
+        job.share(m, static_cast<int>(from));
+        const uint32_t steps = __shfl_sync(kAll, s.steps, from);
+        if (gives) {
+          frames[given].x = kGivenBits | deal[rank_g].y;
+          ++given;
+        }
+        if (takes) {
+          parent = from;
+          given = 0;
+          s.node = node;
+          s.sp = 0;
+          s.steps = steps;
+          s.chain_next = kUMax;
+          s.leaf_far = false;
+          s.best = Hit{INFINITY, kUMax};
+          state = kLaneInner;
+          if (node >= 2 * m.num_tri - 1) {
+            bad = true;
+            state = kLaneHelped;
+          } else {
+            load_record(m.bvhnodes, node, s.left, s.right);
+          }
+        }
+        __syncwarp();
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kTailSteps; ++k)
+      if (state == kLaneInner) state = phase_inner(m, r, stack, kStack, s, bad);
+    if (state == kLaneLeaf) state = phase_leaf(m, r, s, bad);
+    if (state == kLaneAscend) state = phase_ascend(m, r, stack, s, bad, NoFold{}, given);
+    // A ray past the step budget that is about to enter a long chain would
+    // hold the kernel's end: it is handed to the team tier, which folds chains
+    // many links at a time.
+    if (state == kLaneInner && s.steps > long_steps && long_chain_at(m, s.node, s.left, s.right))
+      state = kLaneOverflow;
+    if (state == kLaneDone) {
+      if (parent == kUMax) {
+        job.write(out, m, r, s.best);
+        state = kLaneIdle;
+      } else {
+        state = kLaneHelped;
+      }
+    }
+    uint32_t drop = 0;  // lanes whose result is no longer needed
+    if (__any_sync(kAll, state == kLaneJoin)) {
+      uint4 f = make_uint4(0, 0, 0, 0);
+      if (state == kLaneJoin) f = frames[s.sp - 1];
+      const uint32_t helper = f.x & 31u;
+      const int h_state = __shfl_sync(kAll, state, helper);
+      const Hit h_best{__shfl_sync(kAll, s.best.t, helper), __shfl_sync(kAll, s.best.id, helper)};
+      const bool skip = s.best.id != kUMax && __uint_as_float(f.y) > s.best.t;
+      const bool pop = state == kLaneJoin && (skip || h_state == kLaneHelped);
+      drop = __reduce_or_sync(kAll, pop ? 1u << helper : 0u);
+      if (pop) {
+        s.best = pick(Hit{__uint_as_float(f.z), f.w}, s.best);
+        if (!skip) s.best = pick(s.best, h_best);
+        --s.sp;
+        --given;
+        state = kLaneAscend;
+      }
+    }
+    if (__any_sync(kAll, state == kLaneOverflow)) {
+      // the whole ray goes, whichever of its lanes ran into it
+      uint32_t over = __ballot_sync(kAll, state == kLaneOverflow);
+      for (;;) {
+        const bool up = (over >> lane & 1u) && parent != kUMax;
+        const uint32_t more = over | __reduce_or_sync(kAll, up ? 1u << (parent & 31u) : 0u);
+        if (more == over) break;
+        over = more;
+      }
+      if ((over >> lane & 1u) && parent == kUMax)
+        parked.rays[static_cast<size_t>(slot) * parked.stride + 1].x = atomicExch(handed, slot);
+      drop |= over;
+    }
+    if (drop != 0u) {  // and with a lane all that help it
+      for (;;) {
+        const bool down = state != kLaneIdle && parent != kUMax && (drop >> (parent & 31u) & 1u);
+        const uint32_t more = drop | __ballot_sync(kAll, down);
+        if (more == drop) break;
+        drop = more;
+      }
+      if (drop >> lane & 1u) {
+        state = kLaneIdle;
+        parent = kUMax;
+        given = 0;
+      }
+    }
+  }
+  if (bad) raise_status(status, kStatusBadIndex);
+}
+
+// Re-casts the work indices list_in[0 .. num) by one block, a thread per ray,
+// with stacks carved from the pool.  cap_fixed == 0 chooses the capacity from
+// the number of rays to process.
 template <typename Job>
-__global__ void __launch_bounds__(kTeamThreads, 4) k_cast_team(Job job, const uint32_t* list_in, const uint32_t* count_in,
-                                                          uint32_t* take,
-                                                          uint32_t* list_out, uint32_t* count_out, uint4* pool,
-                                                          uint64_t pool_frames, uint32_t max_tri, uint32_t* status) {
-  __shared__ float smem[64];
-  __shared__ FoldShared sh[kTeamWarps];
-  __shared__ uint32_t sh_take;
-  job.prepare(smem);
-  pdl_wait();
-  pdl_launch_dependents();
-  __syncthreads();
-  const uint32_t num = *count_in;
-  if (num == 0) return;
-  const uint32_t warp = threadIdx.x / 32;
-  const uint64_t warps = static_cast<uint64_t>(gridDim.x) * kTeamWarps;
-  const uint64_t wid = static_cast<uint64_t>(blockIdx.x) * kTeamWarps + warp;
-  const bool whole = num <= kTeamRays * gridDim.x;
-  const Team tm{whole ? sh : sh + warp, whole ? warp : 0u, whole ? kTeamWarps : 1u, threadIdx.x & 31u, 0u, 0u};
-  uint64_t cap = pool_frames / warps;
-  if (cap > 2ull * max_tri) cap = 2ull * max_tri;
+__device__ __noinline__ void cast_deep(const Job& job, const float* smem, const uint32_t* list_in, uint32_t num,
+                                       uint32_t* list_out, uint32_t* count_out, uint4* pool, uint64_t pool_frames,
+                                       uint32_t cap_fixed, uint32_t max_tri, uint32_t* status) {
+  uint64_t cap = cap_fixed;
+  if (cap == 0) {
+    cap = pool_frames / num;
+    if (cap < 256) cap = 256;
+    const uint64_t cap_max = 2ull * max_tri;  // never more than the deepest possible tree needs
+    if (cap > cap_max) cap = cap_max;
+  }
+  if (cap > pool_frames) cap = pool_frames;
+  uint64_t slots = pool_frames / cap;
+  if (slots > blockDim.x) slots = blockDim.x;
+  const uint32_t slot = threadIdx.x;
+  if (slot >= slots) return;
   uint4 ring[kDeepRing];
   uint32_t lo = 0;
-  const RingStack<kDeepRing> st{ring, pool + wid * cap, &lo};
+  const RingStack<kDeepRing> st{ring, pool + slot * cap, &lo};
   bool bad = false;
-  for (;;) {
-    uint32_t k = 0;
-    if (tm.lane == 0 && tm.rank == 0) k = atomicAdd(take, 1u);
-    if (whole) {
-      if (threadIdx.x == 0) sh_take = k;
-      __syncthreads();
-      k = sh_take;
-      __syncthreads();
-    } else {
-      k = __shfl_sync(kWarpAll, k, 0);
-    }
-    if (k >= num) break;
+  for (uint64_t k = slot; k < num; k += slots) {
     lo = 0;
     const uint32_t w = list_in[k];
     MeshView m{};
@@ -874,15 +1039,144 @@ __global__ void __launch_bounds__(kTeamThreads, 4) k_cast_team(Job job, const ui
     int rc = kStepDone;
     if (trav_begin(m, r, s)) {
       do {
-        rc = trav_step_team(m, r, st, static_cast<uint32_t>(cap), s, bad, tm);
+        rc = trav_step(m, r, st, static_cast<uint32_t>(cap), s, bad);
       } while (rc == kStepContinue);
     }
-    if (tm.rank == 0 && tm.lane == 0) {
-      if (rc == kStepDone) job.write(out, m, r, s.best);
-      else list_out[atomicAdd(count_out, 1u)] = w;
+    if (rc == kStepDone) {
+      job.write(out, m, r, s.best);
+    } else if (list_out) {
+      list_out[atomicAdd(count_out, 1u)] = w;
+    } else {
+      raise_status(status, kStatusStackOverflow);
+      job.write(out, m, r, Hit{INFINITY, kUMax});
     }
   }
   if (bad) raise_status(status, kStatusBadIndex);
+}
+
+// One ray cast by a team.  Every lane keeps the same stack (the ring in its own
+// local memory, the spilled frames at the same addresses of its warp's slice of
+// the pool); a ray whose frames outgrow the slice goes to list_out.
+template <typename Job>
+__device__ __noinline__ void cast_team(const Job& job, const float* smem, uint32_t w, const Team& tm, uint4* slice,
+                                       uint32_t cap, uint32_t* list_out, uint32_t* count_out, bool& bad) {
+  uint4 ring[kDeepRing];
+  uint32_t lo = 0;
+  const RingStack<kDeepRing> st{ring, slice, &lo};
+  MeshView m{};
+  Ray r{};
+  uint32_t out = 0;
+  if (!job.fetch(w, smem, m, r, out)) return;
+  Trav s{};
+  int rc = kStepDone;
+  if (trav_begin(m, r, s)) {
+    do {
+      rc = trav_step_team(m, r, st, cap, s, bad, tm);
+    } while (rc == kStepContinue);
+  }
+  if (tm.rank == 0 && tm.lane == 0) {
+    if (rc == kStepDone) job.write(out, m, r, s.best);
+    else list_out[atomicAdd(count_out, 1u)] = w;
+  }
+}
+
+// The lists and counters of the tiers after the persistent cast.
+struct TailArgs {
+  Parked parked;          // rays for the split tier, in the first half of the pool
+  uint32_t* parked_take;  // of them given out
+  const uint32_t* team_list;
+  const uint32_t* team_count;
+  uint32_t* team_take;
+  uint32_t* deep_list;   // rays whose frames outgrew a team's slice
+  uint32_t* deep_count;  // [0] of them, [1] of those that outgrew the next stack
+  uint32_t* last_list;
+  uint32_t* done;        // blocks that have finished
+  uint4* pool;
+  uint64_t pool_frames;
+  uint32_t max_tri, long_steps;
+  uint32_t* status;
+};
+
+// All tiers after the persistent cast in one launch: the split tier, then the
+// team tier, and the last block to finish casts what is left.  With a kernel for
+// each, an image without such rays paid three more launches: 6 us each of a
+// server's dispatcher thread.
+//
+// A team is a whole block while the rays are few, kTeamRays per block or
+// fewer: then the longest ray sets the kernel's end.  With more, their number
+// does, and each warp takes rays of its own.
+constexpr uint32_t kTeamRays = 8;
+template <typename Job, int kStack>
+__global__ void __launch_bounds__(kTeamThreads, 4) k_cast_tail(Job job, TailArgs a) {
+  __shared__ float smem[64];
+  __shared__ FoldShared sh[kTeamWarps];
+  __shared__ uint2 sh_deal[kTeamThreads];
+  __shared__ uint32_t sh_take, sh_handed;
+  job.prepare(smem);
+  if (threadIdx.x == 0) sh_handed = kUMax;
+  pdl_wait();
+  __syncthreads();
+  const uint32_t parked = min(*a.parked.count, a.parked.capacity), num = *a.team_count;
+  if (parked == 0 && num == 0) return;
+  if (parked != 0) {
+    cast_split<Job, kStack>(job, smem, a.parked, parked, a.parked_take, sh_deal, &sh_handed, a.long_steps, a.status);
+    __syncthreads();
+  }
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31u;
+  // the teams' stacks lie in the pool's second half: parked rays may still be
+  // waiting in the first
+  const uint64_t half = a.pool_frames / 2, warps = static_cast<uint64_t>(gridDim.x) * kTeamWarps;
+  const uint64_t cap64 = min(static_cast<unsigned long long>(half / warps), 2ull * a.max_tri);
+  const uint32_t cap = static_cast<uint32_t>(cap64);
+  uint4* slice = a.pool + half + (static_cast<uint64_t>(blockIdx.x) * kTeamWarps + warp) * cap64;
+  bool bad = false;
+  const Team block{sh, warp, kTeamWarps, lane, 0u, 0u};
+  for (uint32_t i = sh_handed; i != kUMax;) {
+    const uint4* ray = a.parked.rays + static_cast<size_t>(i) * a.parked.stride;
+    const uint32_t w = ray[0].x;
+    i = ray[1].x;
+    cast_team(job, smem, w, block, slice, cap, a.deep_list, a.deep_count, bad);
+  }
+  __syncthreads();
+  if (num <= kTeamRays * gridDim.x) {
+    for (;;) {
+      if (threadIdx.x == 0) sh_take = atomicAdd(a.team_take, 1u);
+      __syncthreads();
+      const uint32_t k = sh_take;
+      __syncthreads();
+      if (k >= num) break;
+      cast_team(job, smem, a.team_list[k], block, slice, cap, a.deep_list, a.deep_count, bad);
+    }
+  } else {
+    const Team alone{sh + warp, 0u, 1u, lane, 0u, 0u};
+    for (;;) {
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(a.team_take, 1u);
+      k = __shfl_sync(kWarpAll, k, 0);
+      if (k >= num) break;
+      cast_team(job, smem, a.team_list[k], alone, slice, cap, a.deep_list, a.deep_count, bad);
+    }
+  }
+  if (bad) raise_status(a.status, kStatusBadIndex);
+  // the last block casts the rays whose frames outgrew a slice (none in a tree
+  // of Morton codes, whose chains are folded), with the pool split over them,
+  // then with unbounded frames
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) sh_take = atomicAdd(a.done, 1u);
+  __syncthreads();
+  if (sh_take != gridDim.x - 1) return;
+  __threadfence();
+  const volatile uint32_t* left = a.deep_count;
+  const uint32_t n2 = left[0];
+  if (n2 == 0) return;
+  cast_deep(job, smem, a.deep_list, n2, a.last_list, a.deep_count + 1, a.pool, a.pool_frames, 0u, a.max_tri, a.status);
+  __threadfence();
+  __syncthreads();
+  const uint32_t n3 = left[1];
+  if (n3 == 0) return;
+  cast_deep(job, smem, a.last_list, n3, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr), a.pool,
+            a.pool_frames, a.max_tri < 2 ? 2u : a.max_tri, a.max_tri, a.status);
 }
 
 // Number of resident blocks of a persistent kernel instantiation on the
@@ -902,44 +1196,83 @@ inline int persistent_grid() {
   return cached[dev];
 }
 
-template <typename Job, int kThreads, int kStack>
-inline void launch_persistent(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t* status) {
-  int grid = persistent_grid<Job, kThreads, kStack>();
-  const uint32_t needed = (job.num_work + kThreads - 1) / kThreads;
-  if (static_cast<uint32_t>(grid) > needed) grid = static_cast<int>(needed);
-  const Tuning t = get_tuning();
-  const PhaseMins mins{t.cast_refill_min, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps};
-  k_cast_persistent<Job, kThreads, kStack><<<grid, kThreads, 0, s>>>(job, sc.counters, sc.list1, sc.counters + 1,
-                                                                     status, mins);
+// Node entries after which a ray is parked: kParkSteps for up to kParkRays rays,
+// kParkMore more for each doubling.  Parked too early, rays crowd the split
+// tier; too late, they hold the persistent cast.  Casts in us by threshold:
+//   16,384 rays on a jittered sphere    24: 136   40: 142   64: 160   96: 185   never: 194
+//   641 x 479 on a torus                40: 177   64: 156   80: 159  112: 184   never: 193
+//   512 x 512 on a deformed torus       40: 286   64: 251   80: 235  112: 240   never: 324
+//   1920 x 1080 on a 2M torus           64: 513   96: 446  112: 419  144: 426   never: 603
+constexpr uint32_t kParkSteps = 24, kParkRays = 16384, kParkMore = 14;
+
+inline uint32_t park_steps(uint32_t num_work) {
+  uint32_t doublings = 0;
+  for (uint32_t n = num_work; n >= 2 * kParkRays; n >>= 1) ++doublings;
+  return kParkSteps + kParkMore * doublings;
 }
 
-// The tiered cast of every work index of `job`: the persistent cast; the
-// team tier for the rays it hands over; for the rare ray whose frames outgrow
-// a warp's slice, the serial tier with the pool split over those rays, then
-// with unbounded frames.  sc.counters (kCastCounterBytes) must be zero on
-// entry: [0] work counter, [1..3] the hand-over counts of tiers 1..3 (lists
-// list1, list2, list1 again), [4] rays taken by the team tier.  The first tier's block size and on-chip stack depth
-// come from the current Tuning (kCastVariants lists the choices).
+// `busy`: the GPU has other work to do beside this cast (a server with requests
+// in flight).  Then the cast's own latency counts for less than the issue slots
+// it takes: warps are filled and nothing is parked, as helpers also search
+// subtrees that turn out not to be needed.  64 requests in flight at once took
+// 4.65 ms so and 5.01 ms with parking.
+template <typename Job, int kThreads, int kStack>
+inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, bool busy,
+                         uint32_t* status) {
+  int grid = persistent_grid<Job, kThreads, kStack>();
+  const uint32_t warps = static_cast<uint32_t>(grid) * (kThreads / 32);
+  // few rays are spread over all warps, so that a warp has fewer phases to run
+  // one after the other and more lanes to help in the split tier: 16,384 rays by
+  // 32, 8, 4, 2 per warp: 135, 126, 131, 134 us.  From about 8 per warp on there
+  // is no gain (65,536 rays by 14: 177 against 171 us for build and cast).
+  const uint32_t share =
+      job.num_work <= 8 * warps && !busy ? (job.num_work + warps - 1) / warps : 32u;
+  const uint32_t needed = ((job.num_work + share - 1) / share + kThreads / 32 - 1) / (kThreads / 32);
+  if (static_cast<uint32_t>(grid) > needed) grid = static_cast<int>(needed);
+  const Tuning t = get_tuning();
+  const PhaseMins mins{t.cast_refill_min, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps,
+                       busy ? kUMax : park_steps(job.num_work), share};
+  TailArgs a;
+  a.parked.rays = static_cast<uint4*>(sc.pool);
+  a.parked.count = sc.counters + 5;
+  a.parked.stride = kStack + 2;
+  const uint64_t room = sc.pool_bytes / 2 / (sizeof(uint4) * a.parked.stride);
+  a.parked.capacity = static_cast<uint32_t>(room < (1u << 20) ? room : (1u << 20));
+  a.parked_take = sc.counters + 6;
+  a.team_list = sc.list1;
+  a.team_count = sc.counters + 1;
+  a.team_take = sc.counters + 4;
+  a.deep_list = sc.list2;
+  a.deep_count = sc.counters + 2;
+  a.last_list = sc.list1;
+  a.done = sc.counters + 7;
+  a.pool = static_cast<uint4*>(sc.pool);
+  a.pool_frames = sc.pool_bytes / kFrameBytes;
+  a.max_tri = max_tri;
+  a.long_steps = t.cast_long_steps;
+  a.status = status;
+  k_cast_persistent<Job, kThreads, kStack><<<grid, kThreads, 0, s>>>(job, sc.counters, sc.list1, sc.counters + 1,
+                                                                     status, mins, a.parked);
+  launch_pdl(k_cast_tail<Job, kStack>, dim3(152 * 4), dim3(kTeamThreads), 0, s, job, a);
+}
+
+// The tiered cast of every work index of `job`: the persistent cast, then one
+// kernel for the rays it hands over (k_cast_tail).  sc.counters
+// (kCastCounterBytes) must be zero on entry: [0] rays taken, [1] rays for the
+// team tier (list1), [2], [3] rays for the two deep casts (list2, list1 again),
+// [4] rays taken by the team tier, [5] rays parked, [6] parked rays taken, [7]
+// blocks done.  The first tier's block size and on-chip stack depth come from
+// the current Tuning (kCastVariants lists the choices).
 template <typename Job>
-inline void cast_job(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, uint32_t* status) {
+inline void cast_job(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, uint32_t* status,
+                     bool busy = false) {
   if (job.num_work == 0) return;
   const Tuning t = get_tuning();
-  if (t.cast_threads == 64 && t.cast_stack == 64) launch_persistent<Job, 64, 64>(s, job, sc, status);
-  else if (t.cast_threads == 256 && t.cast_stack == 64) launch_persistent<Job, 256, 64>(s, job, sc, status);
-  else if (t.cast_threads == 128 && t.cast_stack == 32) launch_persistent<Job, 128, 32>(s, job, sc, status);
-  else if (t.cast_threads == 128 && t.cast_stack == 96) launch_persistent<Job, 128, 96>(s, job, sc, status);
-  else launch_persistent<Job, 128, 64>(s, job, sc, status);
-  const uint64_t pool_frames = sc.pool_bytes / kFrameBytes;
-  uint4* pool = static_cast<uint4*>(sc.pool);
-  const uint32_t deep_grid = 152 * 4;
-  launch_pdl(k_cast_team<Job>, dim3(deep_grid), dim3(kTeamThreads), 0, s, job, sc.list1, sc.counters + 1,
-             sc.counters + 4, sc.list2, sc.counters + 2, pool, pool_frames, max_tri, status);
-  launch_pdl(k_cast_deep<Job>, dim3(deep_grid), dim3(kCastThreads), 0, s, job, sc.list2, sc.counters + 2, sc.list1,
-             sc.counters + 3, pool, pool_frames, 0u, max_tri, status);
-  const uint32_t cap3 = max_tri < 2 ? 2u : max_tri;
-  launch_pdl(k_cast_deep<Job>, dim3(deep_grid), dim3(kCastThreads), 0, s, job, sc.list1, sc.counters + 3,
-             static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr), pool, pool_frames, cap3, max_tri,
-             status);
+  if (t.cast_threads == 64 && t.cast_stack == 64) launch_tiers<Job, 64, 64>(s, job, sc, max_tri, busy, status);
+  else if (t.cast_threads == 256 && t.cast_stack == 64) launch_tiers<Job, 256, 64>(s, job, sc, max_tri, busy, status);
+  else if (t.cast_threads == 128 && t.cast_stack == 32) launch_tiers<Job, 128, 32>(s, job, sc, max_tri, busy, status);
+  else if (t.cast_threads == 128 && t.cast_stack == 96) launch_tiers<Job, 128, 96>(s, job, sc, max_tri, busy, status);
+  else launch_tiers<Job, 128, 64>(s, job, sc, max_tri, busy, status);
 }
 
 }  // namespace dm

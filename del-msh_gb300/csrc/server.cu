@@ -223,7 +223,9 @@ int prepare_mesh(cudaStream_t st, const HostMesh& hm, DevMesh& m, uint32_t kind,
 }
 
 // Enqueues the cast of a request and the download of its results.
-int cast_request(cudaStream_t st, const HostMesh& hm, const DevMesh& m, const dm_request& r, const Slot& sl) {
+// busy: other requests are in flight or queued.
+int cast_request(cudaStream_t st, const HostMesh& hm, const DevMesh& m, const dm_request& r, const Slot& sl,
+                 bool busy) {
   MeshView mv{hm.T, hm.V, m.tri, m.vtx, m.bvh, m.aabb};
   CastScratch cs;
   const uint32_t n = (r.kind == DM_REQ_CAST_RAYS) ? r.num_ray : r.img_w * r.img_h;
@@ -235,11 +237,11 @@ int cast_request(cudaStream_t st, const HostMesh& hm, const DevMesh& m, const dm
     float* dir = sl.d_rays + 3ull * n;
     if (cudaMemcpyAsync(org, r.ray_org, 12ull * n, cudaMemcpyHostToDevice, st) != cudaSuccess) return DM_ERR_CUDA;
     if (cudaMemcpyAsync(dir, r.ray_dir, 12ull * n, cudaMemcpyHostToDevice, st) != cudaSuccess) return DM_ERR_CUDA;
-    launch_cast_rays(st, n, org, dir, mv, o, cs, device_status_word());
+    launch_cast_rays(st, n, org, dir, mv, o, cs, device_status_word(), busy);
   } else {
     if (cudaMemcpyAsync(sl.d_transform, r.transform_ndc2world, 64, cudaMemcpyHostToDevice, st) != cudaSuccess)
       return DM_ERR_CUDA;
-    launch_cast_pixels(st, r.img_w, r.img_h, sl.d_transform, mv, o, cs, device_status_word());
+    launch_cast_pixels(st, r.img_w, r.img_h, sl.d_transform, mv, o, cs, device_status_word(), busy);
   }
   if (r.out_tri && cudaMemcpyAsync(r.out_tri, sl.d_hit, 4ull * n, cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return DM_ERR_CUDA;
@@ -385,6 +387,7 @@ void dispatch_loop(dm_server* S) {
     m->inflight++;
     m->last_use = ++S->use_clock;
     const HostMesh& hm = S->host.at(j->req.mesh_id);
+    const bool busy = !S->inflight.empty() || !S->queue.empty();
     lk.unlock();
     // Only this thread changes mesh state and enqueues work, so the mesh
     // fields below are safe without the lock (the completion thread only touches inflight).
@@ -392,7 +395,7 @@ void dispatch_loop(dm_server* S) {
     int rc = DM_OK;
     if (m->has_last && cudaStreamWaitEvent(st, m->last, 0) != cudaSuccess) rc = DM_ERR_CUDA;
     if (rc == DM_OK) rc = prepare_mesh(st, hm, *m, j->req.kind, j->req.frame, j->req.deform_amplitude, sl, S);
-    if (rc == DM_OK) rc = cast_request(st, hm, *m, j->req, sl);
+    if (rc == DM_OK) rc = cast_request(st, hm, *m, j->req, sl, busy);
     if (rc == DM_OK && cudaEventRecord(m->last, st) != cudaSuccess) rc = DM_ERR_CUDA;
     if (rc == DM_OK && cudaEventRecord(sl.done, st) != cudaSuccess) rc = DM_ERR_CUDA;
     if (rc == DM_OK) {
@@ -679,7 +682,7 @@ int dm_plain_run_trace(dm_server* S, uint32_t n, const dm_request* reqs, const d
       } else {
         carve(m, hm.T, hm.V);
         e = prepare_mesh(sl.stream, hm, m, DM_REQ_BUILD_CAST, r.frame, r.deform_amplitude, sl, nullptr);
-        if (e == DM_OK) e = cast_request(sl.stream, hm, m, r, sl);
+        if (e == DM_OK) e = cast_request(sl.stream, hm, m, r, sl, false);
         cudaFreeAsync(m.block, sl.stream);
       }
       if (cudaStreamSynchronize(sl.stream) != cudaSuccess && e == DM_OK) e = DM_ERR_CUDA;
