@@ -201,6 +201,14 @@ int build_impl(uint64_t stream_ptr, uint32_t T, const uint32_t* tri2vtx, uint32_
   // the size class's choices (autotuned; every choice builds the same tree)
   const dm::BuildTuning bt = dm::build_tuning_for(T);
   const bool try_front = bt.build_path == 0 && T >= 2 && T <= dm::front_max_tri();
+  // small meshes: one block does it all (the height needs the tree-order climb,
+  // and the profile has stages to time)
+  if (bt.build_path == 0 && !height_out && !ev &&
+      dm::launch_build_small(s, T, tri2vtx, num_vtx, vtx2xyz, bvhnodes, aabb, transform_out, tri2morton_out,
+                             idx2tri_out, idx2morton_out, other_end_out, status)) {
+    DM_CUDA(cudaGetLastError());
+    return DM_OK;
+  }
   const bool radix10 = bt.sort_radix == 10 || (bt.sort_radix == 0 && T <= dm::kRadix10MaxKeys);
   const SortLayout& SL = radix10 ? L.sort10 : L.sort8;
   // the front needs only the header zeroed; the separate kernels also their

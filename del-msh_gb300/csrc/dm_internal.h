@@ -346,6 +346,17 @@ void launch_interpolate_bwd(cudaStream_t s, uint32_t img_w, uint32_t img_h, cons
                             const MeshView& m, uint32_t num_vdim, const float* vtx2val, const float* ndc2world,
                             const float* dldw_pix2val, float* dldw_vtx2xyz, float* dldw_vtx2val, uint32_t* status);
 
+// --------------------------------------------------------------- small.cu
+// Largest mesh that one block builds.
+constexpr uint32_t kSmallMaxTri = 4096;
+// The whole build by one block; false (nothing launched) when the mesh is not in
+// its range or the device refuses the shared memory.  The outputs after `aabb`
+// are optional.
+bool launch_build_small(cudaStream_t s, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+                        const float* vtx2xyz, uint32_t* bvhnodes, float* aabb, float* transform_out,
+                        uint32_t* tri2morton_out, uint32_t* idx2tri_out, uint32_t* idx2morton_out,
+                        uint32_t* other_end_out, uint32_t* status);
+
 // -------------------------------------------------------------- octree.cu
 // Quad/oct-trees from the binary radix tree of sorted unique Morton codes.
 size_t octree_scratch_bytes(uint32_t num_idx);
