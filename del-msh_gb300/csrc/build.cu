@@ -288,9 +288,11 @@ __global__ void __launch_bounds__(kThreads) k_morton_tri(uint32_t num_tri, const
 // mortons.cu:8-37 (one code per point) with del-msh-cpu's clamping instead of
 // the device asserts (mortons.rs:171-212).
 __global__ void __launch_bounds__(kThreads) k_vtx2morton(uint32_t n, uint32_t num_dim, const float* __restrict__ vtx2co,
-                                                        const float* __restrict__ transform, uint32_t* __restrict__ out) {
+                                                        const float* __restrict__ transform, bool row_major,
+                                                        uint32_t* __restrict__ out) {
   __shared__ float m[16];
-  if (threadIdx.x < 16) m[threadIdx.x] = (threadIdx.x < num_dim * num_dim + 2 * num_dim + 1) ? transform[threadIdx.x] : 0.f;
+  const uint32_t side = num_dim + 1, at = row_major ? (threadIdx.x % side) * side + threadIdx.x / side : threadIdx.x;
+  if (threadIdx.x < 16) m[threadIdx.x] = threadIdx.x < side * side ? transform[at] : 0.f;
   __syncthreads();
   for (uint32_t i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
     if (num_dim == 3) {
@@ -1404,9 +1406,9 @@ void launch_morton_tri(cudaStream_t s, uint32_t num_tri, const uint32_t* tri2vtx
 }
 
 void launch_vtx2morton(cudaStream_t s, uint32_t n, uint32_t num_dim, const float* vtx2co, const float* transform,
-                       uint32_t* out) {
+                       bool row_major, uint32_t* out) {
   const int grid = grid_for(n, kThreads * 4, 152 * 16);
-  k_vtx2morton<<<grid, kThreads, 0, s>>>(n, num_dim, vtx2co, transform, out);
+  k_vtx2morton<<<grid, kThreads, 0, s>>>(n, num_dim, vtx2co, transform, row_major, out);
 }
 
 void launch_topology(cudaStream_t s, uint32_t n, const uint32_t* idx2morton, const uint32_t* idx2obj,
@@ -1546,9 +1548,11 @@ void launch_refit(cudaStream_t s, uint32_t num_tri, const uint32_t* bvhnodes, co
 constexpr uint32_t kSpineWalk = 64;
 
 __global__ void __launch_bounds__(kThreads) k_refit_ends(uint32_t num_tri, const uint32_t* __restrict__ bn,
-                                                         uint32_t* __restrict__ other_end, uint32_t* hdr) {
+                                                         uint32_t* __restrict__ other_end, uint32_t* hdr,
+                                                         uint32_t* zero_flags) {
   const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t nb = num_tri - 1, num_node = 2 * num_tri - 1;
+  if (zero_flags != nullptr && i < num_tri) zero_flags[i] = 0u;
   if (i >= nb) return;
   const uint32_t p = __ldg(bn + 3ull * i), c0 = __ldg(bn + 3ull * i + 1), c1 = __ldg(bn + 3ull * i + 2);
   bool bad = c0 >= num_node || c1 >= num_node;
@@ -1591,7 +1595,7 @@ __global__ void __launch_bounds__(kThreads) k_refit_ends(uint32_t num_tri, const
 
 void launch_refit_any_tree(cudaStream_t s, uint32_t num_tri, const uint32_t* bvhnodes, const uint32_t* tri2vtx,
                            uint32_t num_vtx, const float* vtx2xyz0, const float* vtx2xyz1, float* aabb,
-                           uint32_t* other_end, uint32_t* flags, uint32_t* status) {
+                           uint32_t* other_end, uint32_t* flags, bool zero_flags, uint32_t* status) {
   if (num_tri == 0) return;
   if (num_tri == 1) {  // a single leaf: nothing to climb or query
     launch_refit(s, num_tri, bvhnodes, tri2vtx, num_vtx, vtx2xyz0, vtx2xyz1, aabb, flags, nullptr, status);
@@ -1599,8 +1603,8 @@ void launch_refit_any_tree(cudaStream_t s, uint32_t num_tri, const uint32_t* bvh
   }
   uint32_t* hdr = flags + refit_queue_offset(num_tri);
   cudaMemsetAsync(hdr, 0, kRefitQueueHdr * sizeof(uint32_t), s);
-  const uint32_t grid = (num_tri - 1 + kThreads - 1) / kThreads;
-  k_refit_ends<<<grid, kThreads, 0, s>>>(num_tri, bvhnodes, other_end, hdr);
+  const uint32_t grid = (num_tri + kThreads - 1) / kThreads;
+  k_refit_ends<<<grid, kThreads, 0, s>>>(num_tri, bvhnodes, other_end, hdr, zero_flags ? flags : nullptr);
   launch_refit_windowed(s, num_tri, Segments{}, num_vtx, bvhnodes, other_end, tri2vtx, vtx2xyz0, vtx2xyz1, aabb,
                         flags, nullptr, status, nullptr, /*header_ready=*/true);
   launch_refit(s, num_tri, bvhnodes, tri2vtx, num_vtx, vtx2xyz0, vtx2xyz1, aabb, flags, nullptr, status, hdr + 1);

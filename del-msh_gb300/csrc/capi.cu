@@ -340,10 +340,11 @@ size_t refit_any_scratch_bytes(uint32_t T) {
 }
 
 int refit_any(cudaStream_t s, uint32_t T, const uint32_t* bvhnodes, const uint32_t* tri2vtx, uint32_t V,
-              const float* vtx0, const float* vtx1, float* aabb, void* scratch) {
+              const float* vtx0, const float* vtx1, float* aabb, void* scratch, bool zero_flags) {
   uint32_t* other_end = static_cast<uint32_t*>(scratch);
   uint32_t* flags = at<uint32_t>(scratch, refit_any_flags_offset(T));
-  dm::launch_refit_any_tree(s, T, bvhnodes, tri2vtx, V, vtx0, vtx1, aabb, other_end, flags, status_ptr());
+  dm::launch_refit_any_tree(s, T, bvhnodes, tri2vtx, V, vtx0, vtx1, aabb, other_end, flags, zero_flags,
+                            status_ptr());
   DM_CUDA(cudaGetLastError());
   return DM_OK;
 }
@@ -542,14 +543,21 @@ int dm_selftest_bounded_wait(uint64_t stream_ptr, uint32_t polls, void* scratch,
   return DM_OK;
 }
 
-int dm_mortons_vtx2morton_from_vtx2co(uint64_t stream_ptr, uint32_t num_vtx, uint32_t num_dim, const float* vtx2co,
-                                      const float* transform_co2unit, uint32_t* vtx2morton) {
+int dm_mortons_vtx2morton_from_vtx2co_ex(uint64_t stream_ptr, uint32_t num_vtx, uint32_t num_dim, const float* vtx2co,
+                                      const float* transform_co2unit, uint32_t* vtx2morton, uint32_t flags) {
+  DM_REQUIRE((flags & ~(DM_MATRIX_ROW_MAJOR | DM_DEFINE_OUTPUT)) == 0, "unknown flags 0x%x", flags);
   DM_REQUIRE(num_dim == 2 || num_dim == 3, "num_dim must be 2 or 3 (got %u)", num_dim);
   DM_REQUIRE(transform_co2unit && vtx2morton && (vtx2co || num_vtx == 0), "NULL argument");
   if (num_vtx == 0) return DM_OK;
-  dm::launch_vtx2morton(as_stream(stream_ptr), num_vtx, num_dim, vtx2co, transform_co2unit, vtx2morton);
+  dm::launch_vtx2morton(as_stream(stream_ptr), num_vtx, num_dim, vtx2co, transform_co2unit,
+                        (flags & DM_MATRIX_ROW_MAJOR) != 0, vtx2morton);
   DM_CUDA(cudaGetLastError());
   return DM_OK;
+}
+
+int dm_mortons_vtx2morton_from_vtx2co(uint64_t stream_ptr, uint32_t num_vtx, uint32_t num_dim, const float* vtx2co,
+                                      const float* transform_co2unit, uint32_t* vtx2morton) {
+  return dm_mortons_vtx2morton_from_vtx2co_ex(stream_ptr, num_vtx, num_dim, vtx2co, transform_co2unit, vtx2morton, 0);
 }
 
 size_t dm_array1d_argsort_scratch_bytes(uint32_t n) { return sort_layout(n, 4, 4).total; }
@@ -601,13 +609,23 @@ int dm_bvhnode2aabb_update_aabb(uint64_t stream_ptr, uint32_t num_bvhnode, float
     DM_CUDA(cudaGetLastError());
     return DM_OK;
   }
+  return dm_bvhnode2aabb_update_aabb_fresh(stream_ptr, num_bvhnode, bvhnode2aabb, bvhnodes, num_elem, elem2vtx,
+                                           num_vtx,
+                                           vtx2xyz0, vtx2xyz1, nullptr, 0);
+}
+
+int dm_bvhnode2aabb_update_aabb_fresh(uint64_t stream_ptr, uint32_t num_bvhnode, float* bvhnode2aabb,
+                                      const uint32_t* bvhnodes, uint32_t num_elem, const uint32_t* elem2vtx,
+                                      uint32_t num_vtx, const float* vtx2xyz0, const float* vtx2xyz1, void* scratch,
+                                      size_t scratch_bytes) {
+  if (int e = check_mesh(num_elem, elem2vtx, num_vtx, vtx2xyz0)) return e;
+  DM_REQUIRE(num_bvhnode == 2 * num_elem - 1, "num_bvhnode (%u) must be 2*num_elem-1 (%u)", num_bvhnode,
+             2 * num_elem - 1);
+  DM_REQUIRE(bvhnode2aabb && bvhnodes, "NULL argument");
+  cudaStream_t s = as_stream(stream_ptr);
   Scratch sc;
-  bool fresh = false;
-  const size_t need = refit_any_scratch_bytes(num_elem);
-  if (int e = sc.acquire(nullptr, 0, need, s, &fresh)) return e;
-  DM_CUDA(cudaMemsetAsync(static_cast<unsigned char*>(sc.ptr) + refit_any_flags_offset(num_elem), 0,
-                          size_t{4} * num_elem, s));
-  return refit_any(s, num_elem, bvhnodes, elem2vtx, num_vtx, vtx2xyz0, vtx2xyz1, bvhnode2aabb, sc.ptr);
+  if (int e = sc.acquire(scratch, scratch_bytes, refit_any_scratch_bytes(num_elem), s, nullptr)) return e;
+  return refit_any(s, num_elem, bvhnodes, elem2vtx, num_vtx, vtx2xyz0, vtx2xyz1, bvhnode2aabb, sc.ptr, true);
 }
 
 size_t dm_bvhnode2aabb_update_aabb_scratch_bytes(uint32_t num_elem) { return refit_any_scratch_bytes(num_elem); }
@@ -623,7 +641,7 @@ int dm_bvhnode2aabb_update_aabb_ex(uint64_t stream_ptr, uint32_t num_bvhnode, fl
   const size_t need = refit_any_scratch_bytes(num_elem);
   DM_REQUIRE(scratch_bytes >= need, "scratch of %zu bytes is below the %zu needed", scratch_bytes, need);
   return refit_any(as_stream(stream_ptr), num_elem, bvhnodes, elem2vtx, num_vtx, vtx2xyz0, vtx2xyz1, bvhnode2aabb,
-                   scratch);
+                   scratch, false);
 }
 
 size_t dm_trimesh3_build_scratch_bytes(uint32_t num_tri) { return build_layout(num_tri).total; }
@@ -662,10 +680,11 @@ int dm_trimesh3_build_profiled(uint64_t stream_ptr, uint32_t num_tri, const uint
 
 size_t dm_cast_scratch_bytes(uint32_t num_ray, uint32_t num_tri) { return dm::cast_scratch_bytes(num_ray, num_tri); }
 
-int dm_pix2tri_by_raycast(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, uint32_t* pix2tri, float* pix2t,
+int dm_pix2tri_by_raycast_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, uint32_t* pix2tri, float* pix2t,
                           uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
                           const uint32_t* bvhnodes, const float* bvhnode2aabb, const float* transform_ndc2world,
-                          void* scratch, size_t scratch_bytes) {
+                          void* scratch, size_t scratch_bytes, uint32_t flags) {
+  DM_REQUIRE((flags & ~(DM_MATRIX_ROW_MAJOR | DM_DEFINE_OUTPUT)) == 0, "unknown flags 0x%x", flags);
   if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
   DM_REQUIRE(bvhnodes && bvhnode2aabb && transform_ndc2world && pix2tri, "NULL argument");
   const uint64_t num_pix = static_cast<uint64_t>(img_w) * img_h;
@@ -682,9 +701,20 @@ int dm_pix2tri_by_raycast(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, u
   DM_CUDA(cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, s));
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb};
   dm::CastOut o{pix2tri, pix2t, nullptr};
-  dm::launch_cast_pixels(s, img_w, img_h, transform_ndc2world, m, o, cs, status_ptr());
+  dm::Camera cam;
+  cam.device = transform_ndc2world;
+  cam.row_major = (flags & DM_MATRIX_ROW_MAJOR) != 0;
+  dm::launch_cast_pixels(s, img_w, img_h, cam, m, o, cs, status_ptr());
   DM_CUDA(cudaGetLastError());
   return DM_OK;
+}
+
+int dm_pix2tri_by_raycast(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, uint32_t* pix2tri, float* pix2t,
+                          uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
+                          const uint32_t* bvhnodes, const float* bvhnode2aabb, const float* transform_ndc2world,
+                          void* scratch, size_t scratch_bytes) {
+  return dm_pix2tri_by_raycast_ex(stream_ptr, img_w, img_h, pix2tri, pix2t, num_tri, tri2vtx, num_vtx, vtx2xyz,
+                                  bvhnodes, bvhnode2aabb, transform_ndc2world, scratch, scratch_bytes, 0);
 }
 
 int dm_search_bvh3_first_intersection_ray(uint64_t stream_ptr, uint32_t num_ray, const float* ray_org,
@@ -709,19 +739,50 @@ int dm_search_bvh3_first_intersection_ray(uint64_t stream_ptr, uint32_t num_ray,
   return DM_OK;
 }
 
-int dm_pix2depth_update(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, float* pix2depth,
+int dm_pix2depth_update_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, float* pix2depth,
                         const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
-                        const float* vtx2xyz, const float* transform_ndc2world, void* scratch, size_t scratch_bytes) {
+                        const float* vtx2xyz, const float* transform_ndc2world, void* scratch, size_t scratch_bytes, uint32_t flags) {
+  DM_REQUIRE((flags & ~(DM_MATRIX_ROW_MAJOR | DM_DEFINE_OUTPUT)) == 0, "unknown flags 0x%x", flags);
   if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
   DM_REQUIRE(static_cast<uint64_t>(img_w) * img_h <= kMaxElems, "image of %u x %u pixels is too large", img_w, img_h);
   DM_REQUIRE(pix2depth && pix2tri && transform_ndc2world, "NULL argument");
   cudaStream_t s = as_stream(stream_ptr);
-  Scratch sc;
-  if (int e = sc.acquire(scratch, scratch_bytes, dm_render_scratch_bytes(), s, nullptr)) return e;
-  float* world2ndc = static_cast<float*>(sc.ptr);
-  dm::launch_inverse4(s, transform_ndc2world, world2ndc, status_ptr());
+  if (scratch) {  // not needed any more, but checked as ever
+    Scratch sc;
+    if (int e = sc.acquire(scratch, scratch_bytes, dm_render_scratch_bytes(), s, nullptr)) return e;
+  }
+  const bool row_major = (flags & DM_MATRIX_ROW_MAJOR) != 0, define = (flags & DM_DEFINE_OUTPUT) != 0;
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, nullptr, nullptr};
-  dm::launch_pix2depth(s, img_w, img_h, pix2depth, pix2tri, m, transform_ndc2world, world2ndc, status_ptr());
+  dm::launch_pix2depth(s, img_w, img_h, pix2depth, pix2tri, m, transform_ndc2world, row_major, define, status_ptr());
+  DM_CUDA(cudaGetLastError());
+  return DM_OK;
+}
+
+int dm_pix2depth_update(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, float* pix2depth,
+                        const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+                        const float* vtx2xyz, const float* transform_ndc2world, void* scratch, size_t scratch_bytes) {
+  return dm_pix2depth_update_ex(stream_ptr, img_w, img_h, pix2depth, pix2tri, num_tri, tri2vtx, num_vtx, vtx2xyz,
+                                transform_ndc2world, scratch, scratch_bytes, 0);
+}
+
+int dm_pix2depth_bwd_wrt_vtx2xyz_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, float* dldw_vtx2xyz,
+                                 const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+                                 const float* vtx2xyz, const float* dldw_pix2depth, const float* transform_ndc2world,
+                                 void* scratch, size_t scratch_bytes, uint32_t flags) {
+  DM_REQUIRE((flags & ~(DM_MATRIX_ROW_MAJOR | DM_DEFINE_OUTPUT)) == 0, "unknown flags 0x%x", flags);
+  if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
+  DM_REQUIRE(static_cast<uint64_t>(img_w) * img_h <= kMaxElems, "image of %u x %u pixels is too large", img_w, img_h);
+  DM_REQUIRE(dldw_vtx2xyz && pix2tri && dldw_pix2depth && transform_ndc2world, "NULL argument");
+  cudaStream_t s = as_stream(stream_ptr);
+  if (scratch) {  // not needed any more, but checked as ever
+    Scratch sc;
+    if (int e = sc.acquire(scratch, scratch_bytes, dm_render_scratch_bytes(), s, nullptr)) return e;
+  }
+  const bool row_major = (flags & DM_MATRIX_ROW_MAJOR) != 0, define = (flags & DM_DEFINE_OUTPUT) != 0;
+  dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, nullptr, nullptr};
+  if (define) DM_CUDA(cudaMemsetAsync(dldw_vtx2xyz, 0, 12 * static_cast<size_t>(num_vtx), s));
+  dm::launch_pix2depth_bwd(s, img_w, img_h, dldw_vtx2xyz, pix2tri, m, dldw_pix2depth, transform_ndc2world, row_major,
+                           status_ptr());
   DM_CUDA(cudaGetLastError());
   return DM_OK;
 }
@@ -730,26 +791,16 @@ int dm_pix2depth_bwd_wrt_vtx2xyz(uint64_t stream_ptr, uint32_t img_w, uint32_t i
                                  const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
                                  const float* vtx2xyz, const float* dldw_pix2depth, const float* transform_ndc2world,
                                  void* scratch, size_t scratch_bytes) {
-  if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
-  DM_REQUIRE(static_cast<uint64_t>(img_w) * img_h <= kMaxElems, "image of %u x %u pixels is too large", img_w, img_h);
-  DM_REQUIRE(dldw_vtx2xyz && pix2tri && dldw_pix2depth && transform_ndc2world, "NULL argument");
-  cudaStream_t s = as_stream(stream_ptr);
-  Scratch sc;
-  if (int e = sc.acquire(scratch, scratch_bytes, dm_render_scratch_bytes(), s, nullptr)) return e;
-  float* world2ndc = static_cast<float*>(sc.ptr);
-  dm::launch_inverse4(s, transform_ndc2world, world2ndc, status_ptr());
-  dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, nullptr, nullptr};
-  dm::launch_pix2depth_bwd(s, img_w, img_h, dldw_vtx2xyz, pix2tri, m, dldw_pix2depth, transform_ndc2world, world2ndc,
-                           status_ptr());
-  DM_CUDA(cudaGetLastError());
-  return DM_OK;
+  return dm_pix2depth_bwd_wrt_vtx2xyz_ex(stream_ptr, img_w, img_h, dldw_vtx2xyz, pix2tri, num_tri, tri2vtx, num_vtx,
+                                         vtx2xyz, dldw_pix2depth, transform_ndc2world, scratch, scratch_bytes, 0);
 }
 
 size_t dm_render_scratch_bytes(void) { return 256; }
 
-int dm_pix2tri_interpolate(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
+int dm_pix2tri_interpolate_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
                            uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
-                           uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world, float* pix2val) {
+                           uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world, float* pix2val, uint32_t flags) {
+  DM_REQUIRE((flags & ~(DM_MATRIX_ROW_MAJOR | DM_DEFINE_OUTPUT)) == 0, "unknown flags 0x%x", flags);
   if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
   DM_REQUIRE(static_cast<uint64_t>(img_w) * img_h * (num_vdim ? num_vdim : 1) <= (uint64_t{1} << 32) - 1,
              "image of %u x %u x %u values is too large", img_w, img_h, num_vdim);
@@ -757,7 +808,38 @@ int dm_pix2tri_interpolate(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, 
   DM_REQUIRE(pix2tri && vtx2val && transform_ndc2world && pix2val, "NULL argument");
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, nullptr, nullptr};
   dm::launch_interpolate(as_stream(stream_ptr), img_w, img_h, pix2tri, m, num_vdim, vtx2val, transform_ndc2world,
-                         pix2val, status_ptr());
+                         (flags & DM_MATRIX_ROW_MAJOR) != 0, pix2val, status_ptr());
+  DM_CUDA(cudaGetLastError());
+  return DM_OK;
+}
+
+int dm_pix2tri_interpolate(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
+                           uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
+                           uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world, float* pix2val) {
+  return dm_pix2tri_interpolate_ex(stream_ptr, img_w, img_h, pix2tri, num_tri, tri2vtx, num_vtx, vtx2xyz, num_vdim,
+                                   vtx2val, transform_ndc2world, pix2val, 0);
+}
+
+int dm_pix2tri_interpolate_bwd_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
+                               uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
+                               uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world,
+                               const float* dldw_pix2val, float* dldw_vtx2xyz, float* dldw_vtx2val, uint32_t flags) {
+  DM_REQUIRE((flags & ~(DM_MATRIX_ROW_MAJOR | DM_DEFINE_OUTPUT)) == 0, "unknown flags 0x%x", flags);
+  if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
+  DM_REQUIRE(static_cast<uint64_t>(img_w) * img_h * (num_vdim ? num_vdim : 1) <= (uint64_t{1} << 32) - 1,
+             "image of %u x %u x %u values is too large", img_w, img_h, num_vdim);
+  DM_REQUIRE(num_vdim >= 1, "num_vdim must be >= 1");
+  DM_REQUIRE(pix2tri && vtx2val && transform_ndc2world && dldw_pix2val && dldw_vtx2xyz && dldw_vtx2val,
+             "NULL argument");
+  dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, nullptr, nullptr};
+  cudaStream_t s = as_stream(stream_ptr);
+  if (flags & DM_DEFINE_OUTPUT) {
+    DM_CUDA(cudaMemsetAsync(dldw_vtx2xyz, 0, 12 * static_cast<size_t>(num_vtx), s));
+    DM_CUDA(cudaMemsetAsync(dldw_vtx2val, 0, 4 * static_cast<size_t>(num_vtx) * num_vdim, s));
+  }
+  dm::launch_interpolate_bwd(s, img_w, img_h, pix2tri, m, num_vdim, vtx2val, transform_ndc2world,
+                             (flags & DM_MATRIX_ROW_MAJOR) != 0, dldw_pix2val, dldw_vtx2xyz, dldw_vtx2val,
+                             status_ptr());
   DM_CUDA(cudaGetLastError());
   return DM_OK;
 }
@@ -766,17 +848,9 @@ int dm_pix2tri_interpolate_bwd(uint64_t stream_ptr, uint32_t img_w, uint32_t img
                                uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
                                uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world,
                                const float* dldw_pix2val, float* dldw_vtx2xyz, float* dldw_vtx2val) {
-  if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
-  DM_REQUIRE(static_cast<uint64_t>(img_w) * img_h * (num_vdim ? num_vdim : 1) <= (uint64_t{1} << 32) - 1,
-             "image of %u x %u x %u values is too large", img_w, img_h, num_vdim);
-  DM_REQUIRE(num_vdim >= 1, "num_vdim must be >= 1");
-  DM_REQUIRE(pix2tri && vtx2val && transform_ndc2world && dldw_pix2val && dldw_vtx2xyz && dldw_vtx2val,
-             "NULL argument");
-  dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, nullptr, nullptr};
-  dm::launch_interpolate_bwd(as_stream(stream_ptr), img_w, img_h, pix2tri, m, num_vdim, vtx2val, transform_ndc2world,
-                             dldw_pix2val, dldw_vtx2xyz, dldw_vtx2val, status_ptr());
-  DM_CUDA(cudaGetLastError());
-  return DM_OK;
+  return dm_pix2tri_interpolate_bwd_ex(stream_ptr, img_w, img_h, pix2tri, num_tri, tri2vtx, num_vtx, vtx2xyz,
+                                       num_vdim, vtx2val, transform_ndc2world, dldw_pix2val, dldw_vtx2xyz,
+                                       dldw_vtx2val, 0);
 }
 
 size_t dm_quad_oct_tree_scratch_bytes(uint32_t num_idx) { return dm::octree_scratch_bytes(num_idx); }
@@ -831,21 +905,33 @@ int dm_quad_oct_tree_aggregate(uint64_t stream_ptr, uint32_t num_idx, uint32_t n
   return DM_OK;
 }
 
-int dm_trimesh3_self_intersection(uint64_t stream_ptr, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+int dm_trimesh3_self_intersection_ex(uint64_t stream_ptr, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
                                   const float* vtx2xyz, const uint32_t* bvhnodes, const float* bvhnode2aabb,
-                                  uint32_t capacity, uint32_t* pairs, float* segments, uint32_t* count) {
+                                  uint32_t capacity, uint32_t* pairs, float* segments, uint32_t* count, void* scratch,
+                                     size_t scratch_bytes) {
   if (int e = check_mesh(num_tri, tri2vtx, num_vtx, vtx2xyz)) return e;
   DM_REQUIRE(bvhnodes && bvhnode2aabb && count && (capacity == 0 || (pairs && segments)), "NULL argument");
   cudaStream_t s = as_stream(stream_ptr);
   Scratch sc;
   const size_t need = dm::self_intersection_scratch_bytes(num_tri);
-  if (int e = sc.acquire(nullptr, 0, need, s, nullptr)) return e;
+  if (int e = sc.acquire(scratch, scratch_bytes, need, s, nullptr)) return e;
   DM_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb};
   if (dm::launch_self_intersection(s, m, capacity, pairs, segments, count, sc.ptr, need, status_ptr()) != 0)
     return fail(DM_ERR_CUDA, "self-intersection round failed: %s", cudaGetErrorString(cudaGetLastError()));
   DM_CUDA(cudaGetLastError());
   return DM_OK;
+}
+
+int dm_trimesh3_self_intersection(uint64_t stream_ptr, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+                                  const float* vtx2xyz, const uint32_t* bvhnodes, const float* bvhnode2aabb,
+                                  uint32_t capacity, uint32_t* pairs, float* segments, uint32_t* count) {
+  return dm_trimesh3_self_intersection_ex(stream_ptr, num_tri, tri2vtx, num_vtx, vtx2xyz, bvhnodes, bvhnode2aabb,
+                                          capacity, pairs, segments, count, nullptr, 0);
+}
+
+size_t dm_trimesh3_self_intersection_scratch_bytes(uint32_t num_tri) {
+  return dm::self_intersection_scratch_bytes(num_tri);
 }
 
 size_t dm_batch_build_scratch_bytes(uint32_t num_mesh, uint32_t total_tri) {

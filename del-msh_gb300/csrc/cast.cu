@@ -5,6 +5,8 @@
 // Pixels are handed out in tiles of 32 (8x4 by default, a tuning choice; 32
 // consecutive work indices = one tile) so that the rays of a warp start close
 // together and walk similar nodes.
+#include <cstring>
+
 #include "dm_traverse.cuh"
 
 namespace dm {
@@ -16,13 +18,18 @@ struct SingleJob {
   uint32_t img_w, img_h, tiles_x, tile_w, tile_h;  // pixel mode
   uint32_t tile_w_log;                              // tile_w is a power of two
   Divider by_tiles_x;
-  const float* t_ndc2world;
+  const float* t_ndc2world;  // device matrix, or nullptr: t_value
+  bool row_major;
+  float t_value[16];
   const float* ray_org;  // ray mode when non-null
   const float* ray_dir;
   CastOut o;
 
   __device__ __forceinline__ void prepare(float* smem) const {
-    if (ray_org == nullptr && threadIdx.x < 16) smem[threadIdx.x] = t_ndc2world[threadIdx.x];
+    const uint32_t t = threadIdx.x;
+    if (ray_org != nullptr || t >= 16) return;
+    if (t_ndc2world != nullptr) smem[t] = t_ndc2world[row_major ? (t & 3u) * 4 + (t >> 2) : t];
+    else smem[t] = t_value[t];
   }
 
   __device__ __forceinline__ bool fetch(uint32_t w, const float* smem, MeshView& mv, Ray& r, uint32_t& out) const {
@@ -87,7 +94,7 @@ void cast_scratch_carve(void* base, uint32_t num_ray, uint32_t num_tri, CastScra
   out->pool_bytes = cast_scratch_bytes(num_ray, num_tri) - 256 - 2 * lst;
 }
 
-void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const float* t_ndc2world, const MeshView& m,
+void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const Camera& camera, const MeshView& m,
                         const CastOut& o, const CastScratch& sc, uint32_t* status, bool busy) {
   SingleJob job{};
   job.m = m;
@@ -101,7 +108,9 @@ void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const fl
   job.by_tiles_x = Divider::make(job.tiles_x);
   const uint32_t tiles_y = (img_h + job.tile_h - 1) / job.tile_h;
   job.num_work = job.tiles_x * tiles_y * 32u;
-  job.t_ndc2world = t_ndc2world;
+  job.t_ndc2world = camera.device;
+  job.row_major = camera.row_major;
+  if (camera.host) memcpy(job.t_value, camera.host, sizeof(job.t_value));
   job.o = o;
   cast_job(s, job, sc, m.num_tri, status, busy);
 }

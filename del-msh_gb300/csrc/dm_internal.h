@@ -43,6 +43,7 @@ void launch_morton_tri(cudaStream_t s, uint32_t num_tri, const uint32_t* tri2vtx
 
 // mortons.cu:8-37 semantics with the CPU's clamping (num_dim 2 or 3).
 void launch_vtx2morton(cudaStream_t s, uint32_t n, uint32_t num_dim, const float* vtx2co, const float* transform,
+                       bool row_major,
                        uint32_t* out);
 
 // bvhnodes_morton.rs:10-50 / bvhnodes_morton.cu:29-72.  other_end (optional,
@@ -133,7 +134,7 @@ void launch_refit_windowed(cudaStream_t s, uint32_t total_tri, const Segments& s
 // left zero).
 void launch_refit_any_tree(cudaStream_t s, uint32_t num_tri, const uint32_t* bvhnodes, const uint32_t* tri2vtx,
                            uint32_t num_vtx, const float* vtx2xyz0, const float* vtx2xyz1, float* aabb,
-                           uint32_t* other_end, uint32_t* flags, uint32_t* status);
+                           uint32_t* other_end, uint32_t* flags, bool zero_flags, uint32_t* status);
 
 // ---------------------------------------------------------------- front.cu
 // Centroids, AABB + fit transform, Morton codes and the four-pass stable
@@ -315,8 +316,16 @@ size_t cast_scratch_bytes(uint32_t num_ray, uint32_t num_tri);
 void cast_scratch_carve(void* base, uint32_t num_ray, uint32_t num_tri, CastScratch* out);
 
 // Pixels of an img_w x img_h image (ray_for_pixel.h) or explicit rays.
+// The ndc->world matrix of a cast: 16 floats in device memory, column-major or
+// row-major, or column-major in host memory, read before the call returns and
+// passed with the launch.
+struct Camera {
+  const float* device = nullptr;
+  bool row_major = false;
+  const float* host = nullptr;
+};
 // busy: the GPU has other work beside this cast (see launch_tiers)
-void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const float* t_ndc2world, const MeshView& m,
+void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const Camera& camera, const MeshView& m,
                         const CastOut& o, const CastScratch& sc, uint32_t* status, bool busy = false);
 void launch_cast_rays(cudaStream_t s, uint32_t num_ray, const float* ray_org, const float* ray_dir,
                       const MeshView& m, const CastOut& o, const CastScratch& sc, uint32_t* status,
@@ -330,21 +339,22 @@ void launch_batch_cast_pixels(cudaStream_t s, const Segments& seg, uint32_t max_
                               uint32_t* status);
 
 // --------------------------------------------------------------- render.cu
-// Consumers of a pix2tri image (see render.cu): world2ndc = inverse(ndc2world)
-// on the device (one thread), depth and attribute interpolation, forward and
-// backward (the backward passes accumulate with atomicAdd).
-void launch_inverse4(cudaStream_t s, const float* m, float* inv, uint32_t* status);
+// Consumers of a pix2tri image (see render.cu): depth and attribute interpolation,
+// forward and backward (the backward passes accumulate with atomicAdd).  The
+// matrix is column-major, or row-major with `row_major`; `define`: every pixel is
+// written.
 void launch_pix2depth(cudaStream_t s, uint32_t img_w, uint32_t img_h, float* pix2depth, const uint32_t* pix2tri,
-                      const MeshView& m, const float* ndc2world, const float* world2ndc, uint32_t* status);
+                      const MeshView& m, const float* ndc2world, bool row_major, bool define, uint32_t* status);
 void launch_pix2depth_bwd(cudaStream_t s, uint32_t img_w, uint32_t img_h, float* dldw_vtx2xyz, const uint32_t* pix2tri,
-                          const MeshView& m, const float* dldw_pix2depth, const float* ndc2world,
-                          const float* world2ndc, uint32_t* status);
+                          const MeshView& m, const float* dldw_pix2depth, const float* ndc2world, bool row_major,
+                          uint32_t* status);
 void launch_interpolate(cudaStream_t s, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri, const MeshView& m,
-                        uint32_t num_vdim, const float* vtx2val, const float* ndc2world, float* pix2val,
-                        uint32_t* status);
+                        uint32_t num_vdim, const float* vtx2val, const float* ndc2world, bool row_major,
+                        float* pix2val, uint32_t* status);
 void launch_interpolate_bwd(cudaStream_t s, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
                             const MeshView& m, uint32_t num_vdim, const float* vtx2val, const float* ndc2world,
-                            const float* dldw_pix2val, float* dldw_vtx2xyz, float* dldw_vtx2val, uint32_t* status);
+                            bool row_major, const float* dldw_pix2val, float* dldw_vtx2xyz, float* dldw_vtx2val,
+                            uint32_t* status);
 
 // --------------------------------------------------------------- small.cu
 // Largest mesh that one block builds.

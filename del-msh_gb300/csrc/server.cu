@@ -239,9 +239,11 @@ int cast_request(cudaStream_t st, const HostMesh& hm, const DevMesh& m, const dm
     if (cudaMemcpyAsync(dir, r.ray_dir, 12ull * n, cudaMemcpyHostToDevice, st) != cudaSuccess) return DM_ERR_CUDA;
     launch_cast_rays(st, n, org, dir, mv, o, cs, device_status_word(), busy);
   } else {
-    if (cudaMemcpyAsync(sl.d_transform, r.transform_ndc2world, 64, cudaMemcpyHostToDevice, st) != cudaSuccess)
-      return DM_ERR_CUDA;
-    launch_cast_pixels(st, r.img_w, r.img_h, sl.d_transform, mv, o, cs, device_status_word(), busy);
+    // the matrix goes with the launch: a copy from pageable memory would hold the
+    // dispatcher for several microseconds
+    Camera cam;
+    cam.host = r.transform_ndc2world;
+    launch_cast_pixels(st, r.img_w, r.img_h, cam, mv, o, cs, device_status_word(), busy);
   }
   if (r.out_tri && cudaMemcpyAsync(r.out_tri, sl.d_hit, 4ull * n, cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return DM_ERR_CUDA;

@@ -9,7 +9,8 @@ from __future__ import annotations
 import torch
 
 from .. import _native
-from ..util_torch import assert_shape_dtype_device, ptr, require_cuda, stream_ptr
+from .._native import MATRIX_ROW_MAJOR
+from ..util_torch import assert_shape_dtype_device, plain, ptr, require_cuda, stream_ptr
 
 
 def make_vtx2morton_from_vtx2co(vtx2co: torch.Tensor, transform_co2unit: torch.Tensor) -> torch.Tensor:
@@ -23,7 +24,6 @@ def make_vtx2morton_from_vtx2co(vtx2co: torch.Tensor, transform_co2unit: torch.T
     Returns:
         vtx2morton: (num_vtx,) uint32
     """
-    vtx2co = vtx2co.detach().contiguous()
     num_vtx, num_dim = vtx2co.shape
     device = vtx2co.device
     assert num_dim == 2 or num_dim == 3
@@ -31,9 +31,9 @@ def make_vtx2morton_from_vtx2co(vtx2co: torch.Tensor, transform_co2unit: torch.T
     assert_shape_dtype_device(transform_co2unit, (num_dim + 1, num_dim + 1), torch.float32, device)
     require_cuda(device)
     vtx2morton = torch.empty((num_vtx,), device=device, dtype=torch.uint32)
-    colmajor = transform_co2unit.detach().T.contiguous()
-    _native.call("dm_mortons_vtx2morton_from_vtx2co", stream_ptr(device), num_vtx, num_dim, ptr(vtx2co),
-                 ptr(colmajor), ptr(vtx2morton))
+    vtx2co, mat = plain(vtx2co), plain(transform_co2unit)
+    _native.call("dm_mortons_vtx2morton_from_vtx2co_ex", stream_ptr(device), num_vtx, num_dim, ptr(vtx2co), ptr(mat),
+                 ptr(vtx2morton), MATRIX_ROW_MAJOR)
     return vtx2morton
 
 
@@ -52,7 +52,8 @@ def make_bvhnodes_from_sorted_mortons(idx2obj: torch.Tensor, idx2morton: torch.T
     assert idx2morton.dtype == torch.uint32 and idx2morton.dim() == 1
     assert idx2obj.shape == idx2morton.shape
     require_cuda(device)
+    idx2obj, idx2morton = plain(idx2obj), plain(idx2morton)
     bvhnodes = torch.empty((n * 2 - 1, 3), device=device, dtype=torch.uint32)
-    _native.call("dm_mortons_make_bvhnodes_from_sorted_mortons", stream_ptr(device), n,
-                 ptr(idx2obj.contiguous()), ptr(idx2morton.contiguous()), ptr(bvhnodes))
+    _native.call("dm_mortons_make_bvhnodes_from_sorted_mortons", stream_ptr(device), n, ptr(idx2obj),
+                 ptr(idx2morton), ptr(bvhnodes))
     return bvhnodes

@@ -11,18 +11,17 @@ from __future__ import annotations
 import torch
 
 from .. import _native
-from ..util_torch import assert_shape_dtype_device, ptr, require_cuda, stream_ptr
-
-
-def _scratch(device) -> torch.Tensor:
-    """Room for the device-side world->ndc matrix, from torch's caching
-    allocator (256-byte aligned)."""
-    return torch.empty((_native.load().dm_render_scratch_bytes(),), dtype=torch.uint8, device=device)
+from .._native import DEFINE_OUTPUT, MATRIX_ROW_MAJOR
+from ..util_torch import assert_shape_dtype_device, plain, ptr, require_cuda, stream_ptr
 
 
 def update(pix2depth: torch.Tensor, pix2tri: torch.Tensor, tri2vtx: torch.Tensor, vtx2xyz: torch.Tensor,
            transform_ndc2world: torch.Tensor):
     """Writes the depth of every pixel into pix2depth (img_h, img_w) float32."""
+    _update(pix2depth, pix2tri, tri2vtx, vtx2xyz, transform_ndc2world, 0)
+
+
+def _update(pix2depth, pix2tri, tri2vtx, vtx2xyz, transform_ndc2world, flags):
     num_tri, num_vtx = tri2vtx.shape[0], vtx2xyz.shape[0]
     img_h, img_w = pix2depth.shape[0], pix2depth.shape[1]
     device = pix2depth.device
@@ -32,16 +31,18 @@ def update(pix2depth: torch.Tensor, pix2tri: torch.Tensor, tri2vtx: torch.Tensor
     assert_shape_dtype_device(vtx2xyz, (num_vtx, 3), torch.float32, device)
     assert_shape_dtype_device(transform_ndc2world, (4, 4), torch.float32, device)
     require_cuda(device)
-    colmajor = transform_ndc2world.T.contiguous()
-    scratch = _scratch(device)
-    _native.call("dm_pix2depth_update", stream_ptr(device), img_w, img_h, ptr(pix2depth), ptr(pix2tri.contiguous()),
-                 num_tri, ptr(tri2vtx.contiguous()), num_vtx, ptr(vtx2xyz.detach().contiguous()), ptr(colmajor),
-                 ptr(scratch), scratch.numel())
+    pix2tri, tri2vtx, vtx2xyz, mat = map(plain, (pix2tri, tri2vtx, vtx2xyz, transform_ndc2world))
+    _native.call("dm_pix2depth_update_ex", stream_ptr(device), img_w, img_h, ptr(pix2depth), ptr(pix2tri), num_tri,
+                 ptr(tri2vtx), num_vtx, ptr(vtx2xyz), ptr(mat), None, 0, MATRIX_ROW_MAJOR | flags)
 
 
 def bwd_wrt_vtx2xyz(dldw_vtx2xyz: torch.Tensor, pix2tri: torch.Tensor, tri2vtx: torch.Tensor, vtx2xyz: torch.Tensor,
                     dldw_pix2depth: torch.Tensor, transform_ndc2world: torch.Tensor):
     """Adds d(depth)/d(vtx2xyz)^T dldw_pix2depth into dldw_vtx2xyz (num_vtx, 3)."""
+    _bwd(dldw_vtx2xyz, pix2tri, tri2vtx, vtx2xyz, dldw_pix2depth, transform_ndc2world, 0)
+
+
+def _bwd(dldw_vtx2xyz, pix2tri, tri2vtx, vtx2xyz, dldw_pix2depth, transform_ndc2world, flags):
     num_tri, num_vtx = tri2vtx.shape[0], vtx2xyz.shape[0]
     img_h, img_w = pix2tri.shape[0], pix2tri.shape[1]
     device = dldw_vtx2xyz.device
@@ -52,12 +53,11 @@ def bwd_wrt_vtx2xyz(dldw_vtx2xyz: torch.Tensor, pix2tri: torch.Tensor, tri2vtx: 
     assert_shape_dtype_device(dldw_pix2depth, (img_h, img_w), torch.float32, device)
     assert_shape_dtype_device(transform_ndc2world, (4, 4), torch.float32, device)
     require_cuda(device)
-    colmajor = transform_ndc2world.T.contiguous()
-    scratch = _scratch(device)
-    _native.call("dm_pix2depth_bwd_wrt_vtx2xyz", stream_ptr(device), img_w, img_h, ptr(dldw_vtx2xyz),
-                 ptr(pix2tri.contiguous()), num_tri, ptr(tri2vtx.contiguous()), num_vtx,
-                 ptr(vtx2xyz.detach().contiguous()), ptr(dldw_pix2depth.contiguous()), ptr(colmajor), ptr(scratch),
-                 scratch.numel())
+    pix2tri, tri2vtx, vtx2xyz, dldw_pix2depth, mat = map(
+        plain, (pix2tri, tri2vtx, vtx2xyz, dldw_pix2depth, transform_ndc2world))
+    _native.call("dm_pix2depth_bwd_wrt_vtx2xyz_ex", stream_ptr(device), img_w, img_h, ptr(dldw_vtx2xyz), ptr(pix2tri),
+                 num_tri, ptr(tri2vtx), num_vtx, ptr(vtx2xyz), ptr(dldw_pix2depth), ptr(mat), None, 0,
+                 MATRIX_ROW_MAJOR | flags)
 
 
 class AutogradFunction(torch.autograd.Function):
@@ -68,8 +68,8 @@ class AutogradFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, vtx2xyz, pix2tri, tri2vtx, transform_ndc2world):
-        out = torch.zeros(tuple(pix2tri.shape), dtype=torch.float32, device=vtx2xyz.device)
-        update(out, pix2tri, tri2vtx, vtx2xyz.detach(), transform_ndc2world)
+        out = torch.empty(tuple(pix2tri.shape), dtype=torch.float32, device=vtx2xyz.device)
+        _update(out, pix2tri, tri2vtx, vtx2xyz, transform_ndc2world, DEFINE_OUTPUT)
         # the camera and the hit map are not differentiated, only replayed
         ctx.save_for_backward(vtx2xyz, pix2tri, tri2vtx, transform_ndc2world)
         return out
@@ -79,8 +79,8 @@ class AutogradFunction(torch.autograd.Function):
         vtx2xyz, pix2tri, tri2vtx, transform_ndc2world = ctx.saved_tensors
         if not ctx.needs_input_grad[0]:
             return None, None, None, None
-        grad_vtx = vtx2xyz.new_zeros(vtx2xyz.shape)
-        bwd_wrt_vtx2xyz(grad_vtx, pix2tri, tri2vtx, vtx2xyz.detach(), grad_depth.contiguous(), transform_ndc2world)
+        grad_vtx = torch.empty(vtx2xyz.shape, dtype=vtx2xyz.dtype, device=vtx2xyz.device)
+        _bwd(grad_vtx, pix2tri, tri2vtx, vtx2xyz, grad_depth, transform_ndc2world, DEFINE_OUTPUT)
         return grad_vtx, None, None, None
 
 

@@ -12,7 +12,7 @@ from __future__ import annotations
 import torch
 
 from .. import _native
-from ..util_torch import assert_shape_dtype_device, ptr, require_cuda, scratch, stream_ptr
+from ..util_torch import assert_shape_dtype_device, plain, ptr, require_cuda, scratch, stream_ptr
 
 
 def make_bvhnodes_bvhnode2aabb(tri2vtx: torch.Tensor, vtx2xyz: torch.Tensor):
@@ -25,18 +25,18 @@ def make_bvhnodes_bvhnode2aabb(tri2vtx: torch.Tensor, vtx2xyz: torch.Tensor):
         bvhnodes: (2*num_tri-1, 3) uint32 - [parent, left, right] per node
         bvhnode2aabb: (2*num_tri-1, 6) float32 - [min xyz, max xyz] per node
     """
-    vtx2xyz = vtx2xyz.detach()
     num_vtx = vtx2xyz.shape[0]
     num_tri = tri2vtx.shape[0]
     device = tri2vtx.device
     assert_shape_dtype_device(tri2vtx, (num_tri, 3), torch.uint32, device)
     assert_shape_dtype_device(vtx2xyz, (num_vtx, 3), torch.float32, device)
     require_cuda(device)
+    tri2vtx, vtx2xyz = plain(tri2vtx), plain(vtx2xyz)
     bvhnodes = torch.empty((2 * num_tri - 1, 3), dtype=torch.uint32, device=device)
     bvhnode2aabb = torch.empty((2 * num_tri - 1, 6), dtype=torch.float32, device=device)
-    scr = scratch(device, _native.load().dm_trimesh3_build_scratch_bytes(num_tri))
-    _native.call("dm_trimesh3_make_bvhnodes_bvhnode2aabb", stream_ptr(device), num_tri, ptr(tri2vtx.contiguous()),
-                 num_vtx, ptr(vtx2xyz.contiguous()), ptr(bvhnodes), ptr(bvhnode2aabb), ptr(scr), scr.numel())
+    scr = scratch(device, _native.size("dm_trimesh3_build_scratch_bytes", num_tri))
+    _native.call("dm_trimesh3_make_bvhnodes_bvhnode2aabb", stream_ptr(device), num_tri, ptr(tri2vtx), num_vtx,
+                 ptr(vtx2xyz), ptr(bvhnodes), ptr(bvhnode2aabb), ptr(scr), scr.numel())
     return bvhnodes, bvhnode2aabb
 
 
@@ -91,9 +91,16 @@ def update_bvhnode2aabb(tri2vtx: torch.Tensor, vtx2xyz0: torch.Tensor, bvhnodes:
     if flags is not None:
         assert flags.dtype == torch.uint32 and flags.numel() >= num_tri - 1
     require_cuda(device)
-    _native.call("dm_bvhnode2aabb_update_aabb", stream_ptr(device), num_bvhnode, ptr(bvhnode2aabb), 0, ptr(bvhnodes),
-                 num_tri, ptr(tri2vtx.contiguous()), num_vtx, ptr(vtx2xyz0.detach().contiguous()),
-                 ptr(None if vtx2xyz1 is None else vtx2xyz1.detach().contiguous()), ptr(flags))
+    tri2vtx, vtx2xyz0, vtx2xyz1 = plain(tri2vtx), plain(vtx2xyz0), plain(vtx2xyz1)
+    if flags is not None:
+        _native.call("dm_bvhnode2aabb_update_aabb", stream_ptr(device), num_bvhnode, ptr(bvhnode2aabb), 0,
+                     ptr(bvhnodes), num_tri, ptr(tri2vtx), num_vtx, ptr(vtx2xyz0), ptr(vtx2xyz1), ptr(flags))
+        return bvhnode2aabb
+    # torch keeps the scratch between calls; the device's own pool gives it back
+    # at every synchronisation, and mapping it again took 0.3 ms a call
+    scr = scratch(device, _native.size("dm_bvhnode2aabb_update_aabb_scratch_bytes", num_tri))
+    _native.call("dm_bvhnode2aabb_update_aabb_fresh", stream_ptr(device), num_bvhnode, ptr(bvhnode2aabb),
+                 ptr(bvhnodes), num_tri, ptr(tri2vtx), num_vtx, ptr(vtx2xyz0), ptr(vtx2xyz1), ptr(scr), scr.numel())
     return bvhnode2aabb
 
 
@@ -116,13 +123,15 @@ def self_intersection(tri2vtx: torch.Tensor, vtx2xyz: torch.Tensor, bvhnodes: to
     assert_shape_dtype_device(bvhnodes, (2 * num_tri - 1, 3), torch.uint32, device)
     assert_shape_dtype_device(bvhnode2aabb, (2 * num_tri - 1, 6), torch.float32, device)
     require_cuda(device)
-    count = torch.zeros((1,), dtype=torch.int32, device=device)
+    tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb = map(plain, (tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb))
+    scr = scratch(device, _native.size("dm_trimesh3_self_intersection_scratch_bytes", num_tri))
+    count = torch.empty((1,), dtype=torch.int32, device=device)  # set by the call
     while True:
         pairs = torch.empty((capacity, 2), dtype=torch.uint32, device=device)
         segs = torch.empty((capacity, 2, 3), dtype=torch.float32, device=device)
-        _native.call("dm_trimesh3_self_intersection", stream_ptr(device), num_tri, ptr(tri2vtx.contiguous()),
-                     num_vtx, ptr(vtx2xyz.detach().contiguous()), ptr(bvhnodes.contiguous()),
-                     ptr(bvhnode2aabb.contiguous()), capacity, ptr(pairs), ptr(segs), ptr(count))
+        _native.call("dm_trimesh3_self_intersection_ex", stream_ptr(device), num_tri, ptr(tri2vtx), num_vtx,
+                     ptr(vtx2xyz), ptr(bvhnodes), ptr(bvhnode2aabb), capacity, ptr(pairs), ptr(segs), ptr(count),
+                     ptr(scr), scr.numel())
         n = int(count.item())
         if n <= capacity:
             return segs[:n], pairs[:n]

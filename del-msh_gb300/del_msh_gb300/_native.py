@@ -21,7 +21,10 @@ _SIGNATURES = {
     "dm_device_status": (i32, [C.POINTER(C.c_uint32), i32]),
     "dm_tuning_get": (i32, [vp]),
     "dm_render_scratch_bytes": (sz, []),
+    "dm_trimesh3_self_intersection_scratch_bytes": (sz, [u32]),
     "dm_trimesh3_self_intersection": (i32, [u64, u32, vp, u32, vp, vp, vp, u32, vp, vp, vp]),
+    "dm_trimesh3_self_intersection_ex":
+        (i32, [u64, u32, vp, u32, vp, vp, vp, u32, vp, vp, vp, vp, sz]),
     "dm_quad_oct_tree_scratch_bytes": (sz, [u32]),
     "dm_quad_oct_tree_bnodes_and_bnode2depth_and_bnode2onode_and_idx2bnode":
         (i32, [u64, u32, vp, u32, u32, vp, vp, vp, vp, vp, sz]),
@@ -29,9 +32,17 @@ _SIGNATURES = {
         (i32, [u64, u32, vp, vp, vp, vp, vp, u32, u32, u32, vp, vp, vp, vp, vp]),
     "dm_quad_oct_tree_aggregate": (i32, [u64, u32, u32, vp, vp, u32, vp, u32, vp]),
     "dm_pix2depth_update": (i32, [u64, u32, u32, vp, vp, u32, vp, u32, vp, vp, vp, sz]),
+    "dm_pix2depth_update_ex":
+        (i32, [u64, u32, u32, vp, vp, u32, vp, u32, vp, vp, vp, sz, u32]),
     "dm_pix2depth_bwd_wrt_vtx2xyz": (i32, [u64, u32, u32, vp, vp, u32, vp, u32, vp, vp, vp, vp, sz]),
+    "dm_pix2depth_bwd_wrt_vtx2xyz_ex":
+        (i32, [u64, u32, u32, vp, vp, u32, vp, u32, vp, vp, vp, vp, sz, u32]),
     "dm_pix2tri_interpolate": (i32, [u64, u32, u32, vp, u32, vp, u32, vp, u32, vp, vp, vp]),
+    "dm_pix2tri_interpolate_ex":
+        (i32, [u64, u32, u32, vp, u32, vp, u32, vp, u32, vp, vp, vp, u32]),
     "dm_pix2tri_interpolate_bwd": (i32, [u64, u32, u32, vp, u32, vp, u32, vp, u32, vp, vp, vp, vp, vp]),
+    "dm_pix2tri_interpolate_bwd_ex":
+        (i32, [u64, u32, u32, vp, u32, vp, u32, vp, u32, vp, vp, vp, vp, vp, u32]),
     "dm_tuning_set": (i32, [vp]),
     "dm_build_classes_set": (i32, [vp, u32]),
     "dm_build_classes_get": (i32, [vp, u32, vp]),
@@ -40,18 +51,24 @@ _SIGNATURES = {
     "dm_selftest_bounded_wait": (i32, [u64, u32, vp, sz]),
     "dm_selftest_bounded_wait_scratch_bytes": (sz, []),
     "dm_mortons_vtx2morton_from_vtx2co": (i32, [u64, u32, u32, vp, vp, vp]),
+    "dm_mortons_vtx2morton_from_vtx2co_ex":
+        (i32, [u64, u32, u32, vp, vp, vp, u32]),
     "dm_array1d_argsort": (i32, [u64, u32, vp, vp, vp, sz]),
     "dm_array1d_argsort_scratch_bytes": (sz, [u32]),
     "dm_mortons_make_bvhnodes_from_sorted_mortons": (i32, [u64, u32, vp, vp, vp]),
     "dm_bvhnode2aabb_update_aabb": (i32, [u64, u32, vp, u32, vp, u32, vp, u32, vp, vp, vp]),
     "dm_bvhnode2aabb_update_aabb_noalloc": (i32, [u64, u32, vp, vp, u32, vp, u32, vp, vp]),
     "dm_bvhnode2aabb_update_aabb_ex": (i32, [u64, u32, vp, vp, u32, vp, u32, vp, vp, vp, sz]),
+    "dm_bvhnode2aabb_update_aabb_fresh":
+        (i32, [u64, u32, vp, vp, u32, vp, u32, vp, vp, vp, sz]),
     "dm_bvhnode2aabb_update_aabb_scratch_bytes": (sz, [u32]),
     "dm_trimesh3_make_bvhnodes_bvhnode2aabb": (i32, [u64, u32, vp, u32, vp, vp, vp, vp, sz]),
     "dm_trimesh3_build_scratch_bytes": (sz, [u32]),
     "dm_trimesh3_build_ex": (i32, [u64, u32, vp, u32, vp, vp, vp, vp, vp, vp, vp, vp, vp, sz]),
     "dm_trimesh3_build_profiled": (i32, [u64, u32, vp, u32, vp, vp, vp, vp, sz, vp]),
     "dm_pix2tri_by_raycast": (i32, [u64, u32, u32, vp, vp, u32, vp, u32, vp, vp, vp, vp, vp, sz]),
+    "dm_pix2tri_by_raycast_ex":
+        (i32, [u64, u32, u32, vp, vp, u32, vp, u32, vp, vp, vp, vp, vp, sz, u32]),
     "dm_search_bvh3_first_intersection_ray": (i32, [u64, u32, vp, vp, vp, vp, vp, u32, vp, u32, vp, vp, vp, vp, sz]),
     "dm_cast_scratch_bytes": (sz, [u32, u32]),
     "dm_batch_trimesh3_build": (i32, [u64, u32, vp, vp, u32, u32, u32, vp, vp, vp, vp, vp, vp, sz]),
@@ -68,6 +85,10 @@ SERVER_FUNCS = ("dm_server_create", "dm_server_register_mesh", "dm_server_submit
 
 # entry points that return a status code
 STATUS_FUNCS = {k for k, (r, _) in _SIGNATURES.items() if r is i32 and k != "dm_device_status"}
+
+
+# flags of the *_ex entry points (include/delmsh_gb300.h)
+MATRIX_ROW_MAJOR, DEFINE_OUTPUT = 1, 2
 
 
 class Tuning(C.Structure):
@@ -175,13 +196,26 @@ def exported_symbols():
     return sorted(set(_SIGNATURES) | set(SERVER_FUNCS))
 
 
+_entries = {}  # entry points of the loaded library by name
+
+
 def call(name: str, *args):
     """Calls a status-returning entry point and raises DelMshError on failure."""
-    L = load()
-    rc = getattr(L, name)(*args)
+    fn = _entries.get(name)
+    if fn is None:
+        fn = _entries[name] = getattr(load(), name)
+    rc = fn(*args)
     if rc != 0:
-        raise DelMshError(name, rc, L.dm_last_error().decode())
+        raise DelMshError(name, rc, load().dm_last_error().decode())
     return rc
+
+
+def size(name: str, *args) -> int:
+    """The value of a *_scratch_bytes entry point."""
+    fn = _entries.get(name)
+    if fn is None:
+        fn = _entries[name] = getattr(load(), name)
+    return fn(*args)
 
 
 def device_status(clear: bool = True) -> int:

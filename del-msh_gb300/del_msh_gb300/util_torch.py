@@ -17,8 +17,12 @@ def require_cuda(device: torch.device):
 
 
 def stream_ptr(device: torch.device) -> int:
-    torch.cuda.set_device(device)
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current stream of a CUDA device, which becomes the current device."""
+    index = device.index
+    if torch.cuda.current_device() != index:
+        torch.cuda.set_device(device)
+        index = torch.cuda.current_device()
+    return torch._C._cuda_getCurrentRawStream(index)
 
 
 def ptr(t):
@@ -27,6 +31,13 @@ def ptr(t):
         return None
     assert t.is_contiguous(), "tensor must be contiguous"
     return t.data_ptr()
+
+
+def plain(t):
+    """The tensor itself when it is contiguous, else a contiguous copy outside
+    autograd.  The caller keeps it until the launch: its address alone does not
+    hold the copy."""
+    return t if t is None or t.is_contiguous() else t.detach().contiguous()
 
 
 def scratch(device: torch.device, nbytes: int) -> torch.Tensor:

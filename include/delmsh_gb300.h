@@ -46,6 +46,13 @@ extern "C" {
 #define DM_ERR_SCRATCH_TOO_SMALL 3
 #define DM_ERR_UNSUPPORTED 4
 
+/* Flags of the *_ex entries.  DM_MATRIX_ROW_MAJOR: the matrix is row-major (as
+ * torch holds it), not column-major.  DM_DEFINE_OUTPUT: the output need not hold
+ * anything before the call: an image gets 0 where the plain entry leaves a pixel
+ * as it is, gradients are set to 0 and not added to. */
+#define DM_MATRIX_ROW_MAJOR 1u
+#define DM_DEFINE_OUTPUT 2u
+
 /* Library version string. */
 const char* dm_version(void);
 
@@ -138,6 +145,10 @@ size_t dm_selftest_bounded_wait_scratch_bytes(void);
 int dm_mortons_vtx2morton_from_vtx2co(uint64_t stream_ptr, uint32_t num_vtx, uint32_t num_dim,
                                       const float* vtx2co, const float* transform_co2unit,
                                       uint32_t* vtx2morton);
+/* The same with flags (DM_MATRIX_ROW_MAJOR, DM_DEFINE_OUTPUT). */
+int dm_mortons_vtx2morton_from_vtx2co_ex(uint64_t stream_ptr, uint32_t num_vtx, uint32_t num_dim,
+                                      const float* vtx2co, const float* transform_co2unit,
+                                      uint32_t* vtx2morton, uint32_t flags);
 
 /* Stable ascending sort of u32 values in place, writing the permutation
  * (jdx2idx[j] = original position of the j-th smallest; ties keep ascending
@@ -178,6 +189,15 @@ int dm_bvhnode2aabb_update_aabb(uint64_t stream_ptr, uint32_t num_bvhnode, float
                                 uint32_t i_bvhnode, const uint32_t* bvhnodes, uint32_t num_elem,
                                 const uint32_t* elem2vtx, uint32_t num_vtx, const float* vtx2xyz0,
                                 const float* vtx2xyz1, uint32_t* flags_scratch);
+
+/* dm_bvhnode2aabb_update_aabb (flags_scratch == NULL form) with caller scratch of
+ * dm_bvhnode2aabb_update_aabb_scratch_bytes(num_elem) bytes, whatever it holds
+ * (or NULL).
+ * Replaces: del-msh-dlpack/src/bvhnode2aabb.rs:15-108 bvhnode2aabb_update_aabb. */
+int dm_bvhnode2aabb_update_aabb_fresh(uint64_t stream_ptr, uint32_t num_bvhnode, float* bvhnode2aabb,
+                                      const uint32_t* bvhnodes, uint32_t num_elem, const uint32_t* elem2vtx,
+                                      uint32_t num_vtx, const float* vtx2xyz0, const float* vtx2xyz1, void* scratch,
+                                      size_t scratch_bytes);
 
 /* dm_bvhnode2aabb_update_aabb (flags_scratch == NULL form) with caller
  * scratch of dm_bvhnode2aabb_update_aabb_scratch_bytes(num_elem) bytes,
@@ -251,6 +271,11 @@ int dm_pix2tri_by_raycast(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, u
                           uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
                           const uint32_t* bvhnodes, const float* bvhnode2aabb, const float* transform_ndc2world,
                           void* scratch, size_t scratch_bytes);
+/* The same with flags (DM_MATRIX_ROW_MAJOR, DM_DEFINE_OUTPUT). */
+int dm_pix2tri_by_raycast_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, uint32_t* pix2tri, float* pix2t,
+                          uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
+                          const uint32_t* bvhnodes, const float* bvhnode2aabb, const float* transform_ndc2world,
+                          void* scratch, size_t scratch_bytes, uint32_t flags);
 
 /* Closest hit of each ray (ray_org, ray_dir f32[num_ray*3]); hit_t and hit_bc
  * (barycentrics 1-u-v, u, v; f32[num_ray*3]) may be NULL.
@@ -284,6 +309,10 @@ size_t dm_render_scratch_bytes(void);
 int dm_pix2depth_update(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, float* pix2depth,
                         const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
                         const float* vtx2xyz, const float* transform_ndc2world, void* scratch, size_t scratch_bytes);
+/* The same with flags (DM_MATRIX_ROW_MAJOR, DM_DEFINE_OUTPUT). */
+int dm_pix2depth_update_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, float* pix2depth,
+                        const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+                        const float* vtx2xyz, const float* transform_ndc2world, void* scratch, size_t scratch_bytes, uint32_t flags);
 
 /* dldw_vtx2xyz += d(pix2depth)/d(vtx2xyz)^T dldw_pix2depth.
  * Replaces: del-msh-dlpack/src/pix2depth.rs:100-189 pix2depth_bwd_wrt_vtx2xyz
@@ -292,6 +321,11 @@ int dm_pix2depth_bwd_wrt_vtx2xyz(uint64_t stream_ptr, uint32_t img_w, uint32_t i
                                  const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
                                  const float* vtx2xyz, const float* dldw_pix2depth, const float* transform_ndc2world,
                                  void* scratch, size_t scratch_bytes);
+/* The same with flags (DM_MATRIX_ROW_MAJOR, DM_DEFINE_OUTPUT). */
+int dm_pix2depth_bwd_wrt_vtx2xyz_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, float* dldw_vtx2xyz,
+                                 const uint32_t* pix2tri, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+                                 const float* vtx2xyz, const float* dldw_pix2depth, const float* transform_ndc2world,
+                                 void* scratch, size_t scratch_bytes, uint32_t flags);
 
 /* pix2val[p] = bc0 vtx2val[i0] + bc1 vtx2val[i1] + bc2 vtx2val[i2] with the
  * barycentric coordinates of the pixel ray on its triangle; 0 on the
@@ -301,6 +335,10 @@ int dm_pix2depth_bwd_wrt_vtx2xyz(uint64_t stream_ptr, uint32_t img_w, uint32_t i
 int dm_pix2tri_interpolate(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
                            uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
                            uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world, float* pix2val);
+/* The same with flags (DM_MATRIX_ROW_MAJOR, DM_DEFINE_OUTPUT). */
+int dm_pix2tri_interpolate_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
+                           uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
+                           uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world, float* pix2val, uint32_t flags);
 
 /* Backward of dm_pix2tri_interpolate: adds to dldw_vtx2xyz (f32[V][3]) and
  * dldw_vtx2val (f32[V][num_vdim]).
@@ -310,6 +348,11 @@ int dm_pix2tri_interpolate_bwd(uint64_t stream_ptr, uint32_t img_w, uint32_t img
                                uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
                                uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world,
                                const float* dldw_pix2val, float* dldw_vtx2xyz, float* dldw_vtx2val);
+/* The same with flags (DM_MATRIX_ROW_MAJOR, DM_DEFINE_OUTPUT). */
+int dm_pix2tri_interpolate_bwd_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h, const uint32_t* pix2tri,
+                               uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx, const float* vtx2xyz,
+                               uint32_t num_vdim, const float* vtx2val, const float* transform_ndc2world,
+                               const float* dldw_pix2val, float* dldw_vtx2xyz, float* dldw_vtx2val, uint32_t flags);
 
 /* Self-intersecting triangle pairs of a mesh through its BVH: for each pair
  * (i, j) (the triangle of the left subtree first) the segment (p0, p1) where
@@ -318,16 +361,25 @@ int dm_pix2tri_interpolate_bwd(uint64_t stream_ptr, uint32_t img_w, uint32_t img
  * pierces the other triangle.  *count (device u32) receives the number of
  * pairs, which may exceed `capacity`, in which case only `capacity` pairs are
  * written (call again with a larger buffer).  The list is unordered.  The
- * search runs depth-first per thread (192-entry node-pair stack; status bit
- * 2 if one overflows) in rounds that rebalance the remaining work; each round
+ * search keeps one 704-entry stack of node pairs per warp (status bit 2 if one
+ * overflows) and runs in rounds that rebalance the remaining work; every fourth
  * reads the next round's size back to the host, so the call synchronizes the
  * stream.  Its working memory (16 MB per million triangles, at least 16 MB)
- * comes from cudaMallocAsync.
+ * comes from cudaMallocAsync, or from the caller in the _ex form.
  * Replaces: del-msh-cpu/src/trimesh3_intersection.rs:86-179
  * search_with_bvh_inside_branch (binding del-msh-numpy/src/mesh_intersection.rs). */
 int dm_trimesh3_self_intersection(uint64_t stream_ptr, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
                                   const float* vtx2xyz, const uint32_t* bvhnodes, const float* bvhnode2aabb,
                                   uint32_t capacity, uint32_t* pairs, float* segments, uint32_t* count);
+
+/* The same with caller scratch of dm_trimesh3_self_intersection_scratch_bytes
+ * bytes (or NULL). */
+int dm_trimesh3_self_intersection_ex(uint64_t stream_ptr, uint32_t num_tri, const uint32_t* tri2vtx, uint32_t num_vtx,
+                                  const float* vtx2xyz, const uint32_t* bvhnodes, const float* bvhnode2aabb,
+                                  uint32_t capacity, uint32_t* pairs, float* segments, uint32_t* count, void* scratch,
+                                     size_t scratch_bytes);
+size_t dm_trimesh3_self_intersection_scratch_bytes(uint32_t num_tri);
+
 
 /* ---- quad/oct-trees from the binary radix tree of sorted unique Morton codes ----
  * Layouts of del-msh-cpu/src/quad_oct_tree.rs: bnodes u32[num_idx-1][3]
