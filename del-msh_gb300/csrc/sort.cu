@@ -225,13 +225,23 @@ __global__ void __launch_bounds__(kThreads, sizeof(KeyT) == 4 ? 4 : 2) k_oneswee
 // memory: after a __syncwarp the slot holds exactly the lanes with that digit
 // (the peers), the lowest of them advances the warp's running count of the
 // digit and clears the slot.  That is about 15 instructions per key against
-// the ~40 of eight ballots, and with 8 keys per thread the pass keeps keys,
-// ranks and values in registers without spilling.  Counts, look-back and
-// write-out are those of k_onesweep.
+// the ~40 of eight ballots.  Counts, look-back and write-out are those of
+// k_onesweep.
+// What bounds it is how many of the waits (keys, look-back, barriers) a
+// multiprocessor has in flight: at two blocks it issued in 28 % of the cycles
+// with half its warps resident.  So a thread holds no more than 40 registers,
+// which with 71 KB of shared memory gives three blocks: ranks within a warp's
+// 256 keys are packed as bytes, values are not loaded before the scatter, and
+// the keys are on their way while the histogram is scanned.  Argsort of 3, 6
+// and 16 million keys: 175, 280, 711 us at two blocks, 157, 238, 519 us here
+// (16 M: 2.0 TB/s of keys and values over the four passes).  Four blocks (the
+// masks' space shared with the values) gave 627 against 610 us in a build of
+// 6 million triangles.
 constexpr int kThreadsM = 512;
 constexpr int kWarpsM = kThreadsM / 32;
 constexpr int kKptM = 8;
 constexpr int kTileM = kThreadsM * kKptM;  // 4096
+static_assert(32 * kKptM <= 256, "ranks are bytes");
 static_assert(kTileM >= kSortTile, "a match-pass tile covers at least a k_onesweep tile (look-back sizing)");
 
 struct SortSmemM {
@@ -274,7 +284,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_m(uint32_t v, uint32_t*
 }
 
 template <bool kIota, int kWindow>
-__global__ void __launch_bounds__(kThreadsM, 2) k_onesweep_match(const uint32_t* __restrict__ keys_in,
+__global__ void __launch_bounds__(kThreadsM, 3) k_onesweep_match(const uint32_t* __restrict__ keys_in,
                                                                const uint32_t* __restrict__ vals_in,
                                                                uint32_t* __restrict__ keys_out,
                                                                uint32_t* __restrict__ vals_out, uint32_t n,
@@ -293,24 +303,21 @@ __global__ void __launch_bounds__(kThreadsM, 2) k_onesweep_match(const uint32_t*
   if (tid == 0) S.tile = atomicAdd(tile_counter, 1u);
   pdl_wait();
   pdl_launch_dependents();
-  const uint32_t gb = block_exclusive_scan_m(tid < kRadix ? __ldg(hist + tid) : 0u, S.scan);  // has __syncthreads
-  if (tid < kRadix) S.gbase[tid] = gb;
+  __syncthreads();
   const uint32_t tile = S.tile;
   const uint32_t tile_base = tile * kTileM;
   const uint32_t wbase = tile_base + static_cast<uint32_t>(warp) * 32u * kKptM;
 
-  uint32_t keys[kKptM], ranks[kKptM], vals[kKptM];
+  uint32_t keys[kKptM];
+  uint32_t ranks[kKptM / 4] = {};  // a warp ranks 256 keys: a byte each
 #pragma unroll
   for (int j = 0; j < kKptM; ++j) {
     const uint32_t idx = wbase + 32u * j + lane;
     keys[j] = idx < n ? keys_in[idx] : 0u;
   }
-#pragma unroll
-  for (int j = 0; j < kKptM; ++j) {
-    const uint32_t idx = wbase + 32u * j + lane;
-    vals[j] = kIota ? idx : (idx < n ? vals_in[idx] : 0u);
-  }
-
+  // the keys are on their way during the scan of the upfront histogram
+  const uint32_t gb = block_exclusive_scan_m(tid < kRadix ? __ldg(hist + tid) : 0u, S.scan);  // has __syncthreads
+  if (tid < kRadix) S.gbase[tid] = gb;
   // Rank inside the warp in (j, lane) order, i.e. input order.
   const uint32_t lt_mask = (1u << lane) - 1u;
   uint32_t* wh = S.whist[warp];
@@ -329,7 +336,7 @@ __global__ void __launch_bounds__(kThreadsM, 2) k_onesweep_match(const uint32_t*
       wm[d] = 0u;
     }
     __syncwarp();
-    ranks[j] = before + __popc(peers & lt_mask);
+    ranks[j / 4] |= (before + __popc(peers & lt_mask)) << (8 * (j % 4));
   }
   __syncthreads();
 
@@ -353,11 +360,12 @@ __global__ void __launch_bounds__(kThreadsM, 2) k_onesweep_match(const uint32_t*
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < kKptM; ++j) {
-    if (wbase + 32u * j + lane < n) {
+    const uint32_t idx = wbase + 32u * j + lane;
+    if (idx < n) {
       const uint32_t dg = (keys[j] >> shift) & (kRadix - 1);
-      const uint32_t pos = S.tstart[dg] + S.whist[warp][dg] + ranks[j];
+      const uint32_t pos = S.tstart[dg] + S.whist[warp][dg] + (ranks[j / 4] >> (8 * (j % 4)) & 255u);
       S.keys[pos] = keys[j];
-      S.vals[pos] = vals[j];
+      S.vals[pos] = kIota ? idx : vals_in[idx];
     }
   }
 
