@@ -230,8 +230,8 @@ __global__ void __launch_bounds__(kThreads) k_batch_topology(uint32_t total_bran
 //            over the cluster, and the fit transform; the centroids wait in
 //            the (still empty) sort buffers
 //   codes    Morton code of every centroid, stored at the triangle's position
-//   4 passes stable LSD radix sort on 8-bit digits: warp ballots rank each
-//            key within its warp (as k_onesweep), per-warp and per-block
+//   4 passes stable LSD radix sort on 8-bit digits: peer masks rank each key
+//            within its warp (as k_onesweep_match), per-warp and per-block
 //            digit counts give every key its output position in the mesh, and
 //            the key is written to the block owning that position
 //   topology Karras branches (topology_node) over the sorted codes, read from
@@ -351,6 +351,19 @@ __device__ __forceinline__ void seg_pass(SegSmem& S, int src, uint32_t shift, ui
   const uint32_t n_w = n_c > wpos ? min(n_c - wpos, chunk) : 0u;
   const uint32_t lt_mask = (1u << lane) - 1u;
   uint16_t* my = S.whist[warp];
+  // Peer masks of this warp, in the buffer that the pass has yet to fill (no
+  // block writes it before the counts' barrier).  Ranking was the second
+  // longest phase with eight ballots a key: 4.5 cycles a key over the four
+  // passes, 2.8 with the masks; 1024 meshes of 64..65536 triangles (9.7
+  // million) 995 -> 885 us.  What is left: topology 8.9 cycles a key, the
+  // scatter 7.6 (two remote stores a key, about one a cycle), fit 3.
+  uint32_t* mask = &S.code[src ^ 1][warp * kRadix];
+  if (n_w > 0) {
+    uint4* z = reinterpret_cast<uint4*>(mask);
+#pragma unroll
+    for (int i = 0; i < kRadix / 4 / 32; ++i) z[i * 32 + lane] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  __syncwarp();
   // rank in (slot, lane) order, i.e. position order; two 16-bit ranks per word
   uint32_t rk[kSegSlots / 2];
 #pragma unroll
@@ -360,10 +373,15 @@ __device__ __forceinline__ void seg_pass(SegSmem& S, int src, uint32_t shift, ui
       const uint32_t p = static_cast<uint32_t>(k) * 32u + lane;
       const bool valid = p < n_w;
       const uint32_t d = valid ? (S.code[src][wpos + p] >> shift) & 0xFFu : 0u;
-      const uint32_t peers = warp_peers(d, valid);
+      if (valid) atomicOr(mask + d, 1u << lane);
+      __syncwarp();
+      const uint32_t peers = valid ? mask[d] : 0u;
       const uint32_t before = valid ? my[d] : 0u;
       __syncwarp();
-      if (valid && lane == __ffs(peers) - 1) my[d] = static_cast<uint16_t>(before + __popc(peers));
+      if (valid && (peers & lt_mask) == 0u) {
+        my[d] = static_cast<uint16_t>(before + __popc(peers));
+        mask[d] = 0u;
+      }
       __syncwarp();
       r = before + __popc(peers & lt_mask);
     }
@@ -406,8 +424,9 @@ __device__ __forceinline__ void seg_pass(SegSmem& S, int src, uint32_t shift, ui
       const uint32_t out = S.off[d] + S.whist[warp][d] + r;
       const uint32_t owner = sp.owner(out), q = out - owner * sp.per;
       if (owner < static_cast<uint32_t>(kC)) {  // always: the counts add up to the mesh
-        SegGroup<kC>::at(&S.code[dst][0], owner)[q] = key;
-        SegGroup<kC>::at(&S.idx[dst][0], owner)[q] = id;
+        SegSmem& to = *SegGroup<kC>::at(&S, owner);
+        to.code[dst][q] = key;
+        to.idx[dst][q] = id;
       }
     }
   }
