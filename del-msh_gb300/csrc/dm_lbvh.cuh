@@ -58,33 +58,39 @@ __device__ __forceinline__ void karras_range_split(uint32_t n, const Codes& c, u
     } else {
       const int dd = __clz(mc1 ^ mc2) - __clz(mc1 ^ mc0);
       const bool up = dd > 0;  // direction d = +1 (else -1)
-      const int delta_min = __clz(mc1 ^ (up ? mc0 : mc2));
+      // more than delta_min = clz(x) leading bits shared <=> the difference is
+      // below x's highest bit (x is not 0 here): one compare per step instead
+      // of a clz, which runs at a fraction of the rate of the compare (k_topology
+      // of 65k, 2M, 6M triangles: 11.2, 45, 146 -> 9.7, 40, 136 us)
+      const uint32_t x = mc1 ^ (up ? mc0 : mc2);
+      const uint32_t below = 0x80000000u >> __clz(x);
       // 32-bit steps: lim is the largest step that stays inside [0, n) in
       // direction d (n < 2^30, so lmax <= 2 (lim + 1) fits), and a step s
       // lands on ib + s or ib - s
-      const uint32_t lim = up ? n - 1 - ib : ib;
+      const uint32_t lim = up ? n - 1 - ib : ib, d = up ? 1u : kUMax;
       uint32_t lmax = 2;
-      while (lmax <= lim && __clz(mc1 ^ c(up ? ib + lmax : ib - lmax)) > delta_min) lmax *= 2;
+      while (lmax <= lim && (mc1 ^ c(ib + lmax * d)) < below) lmax *= 2;
       uint32_t l = 0;
       for (uint32_t t = lmax / 2; t >= 1; t /= 2) {
         const uint32_t s = l + t;
-        if (s <= lim && __clz(mc1 ^ c(up ? ib + s : ib - s)) > delta_min) l = s;
+        if (s <= lim && (mc1 ^ c(ib + s * d)) < below) l = s;
       }
-      const uint32_t j = up ? ib + l : ib - l;
+      const uint32_t j = ib + l * d;
       r0 = up ? ib : j;
       r1 = up ? j : ib;
     }
   }
   isplit = r0;
   const uint32_t mc_start = c(r0);
-  const int common = __clz(mc_start ^ c(r1));
-  if (common != 32) {
+  const uint32_t diff = mc_start ^ c(r1);
+  if (diff != 0u) {
+    const uint32_t below = 0x80000000u >> __clz(diff);
     uint32_t step = r1 - r0;
     while (step > 1) {
       step = (step + 1) / 2;
       const uint32_t cand = isplit + step;
       if (cand >= r1) continue;
-      if (__clz(mc_start ^ c(cand)) > common) isplit = cand;
+      if ((mc_start ^ c(cand)) < below) isplit = cand;
     }
   }
 }
