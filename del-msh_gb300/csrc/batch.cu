@@ -667,6 +667,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_seg_classify(Segments seg, u
 
 
 struct BatchJob {
+  static constexpr uint32_t kRefillHalves = 3;
   uint32_t num_work;
   Segments seg;
   const uint32_t* tri2vtx;

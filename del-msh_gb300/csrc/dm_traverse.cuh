@@ -394,6 +394,7 @@ constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 //   __device__ void share(MeshView& m, int from) const;
 //                                                   m becomes that of lane `from` (all lanes call it)
 //   __device__ void write(uint32_t out, const MeshView& m, const Ray& r, const Hit& h) const;
+//   kRefillHalves                                   halves of cast_refill_min at which a warp takes rays
 
 // Thresholds of the phased loop: a phase runs when at least this many lanes
 // of the warp wait for it, or when nothing else can run.
@@ -1230,7 +1231,14 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   const uint32_t needed = ((job.num_work + share - 1) / share + kThreads / 32 - 1) / (kThreads / 32);
   if (static_cast<uint32_t>(grid) > needed) grid = static_cast<int>(needed);
   const Tuning t = get_tuning();
-  const PhaseMins mins{t.cast_refill_min, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps,
+  // One mesh takes rays as soon as a quarter of a warp is idle; a batch, whose
+  // fetch reads a dozen words of tables and a matrix per ray, waits for half as
+  // many again.  Threshold 12 and 8: 2M triangles at 1920 x 1080 458 and 438 us,
+  // 500 thousand at 512 x 512 243 and 222 us, but the batch 1232 and 1267 us
+  // (at 9, 8, 6 for a mesh and 13, 12, 9 for the batch: 437, 438, 441; 1230,
+  // 1231, 1253 us).
+  const uint32_t refill = min(t.cast_refill_min * Job::kRefillHalves / 2u, 32u);
+  const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps,
                        busy ? kUMax : park_steps(job.num_work), share};
   TailArgs a;
   a.parked.rays = static_cast<uint4*>(sc.pool);
