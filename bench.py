@@ -43,12 +43,12 @@ import numpy as np  # noqa: E402
 METRIC = "rays/s (LBVH build + cast per step)"
 UNIT = "rays/s"
 IMG_W, IMG_H = 1920, 1080
-# kernels of this repo launched per single-mesh step: build = centroid AABB,
-# Morton, 4 sort passes, topology, 6 refit kernels (window, superblock, the
-# two crossing-branch kernels, and the tree-order climb's two, which exit at
-# once without NaN); cast = persistent traversal + the team tier + 2 serial
-# overflow tiers (the last three exit at once when their lists are empty)
-KERNELS_PER_STEP = 17
+# kernels of this repo launched per single-mesh step: build = the cooperative
+# front (centroids, codes, sort), topology, 6 refit kernels (window,
+# superblock, the two crossing-branch kernels, and the tree-order climb's two,
+# which exit at once without NaN); cast = the counters, the persistent
+# traversal, and the kernel that finishes the long rays
+KERNELS_PER_STEP = 11
 NDIV = 1024
 SEED = 0
 L2_FLUSH_BYTES = 256 << 20

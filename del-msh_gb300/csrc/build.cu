@@ -312,17 +312,26 @@ __global__ void __launch_bounds__(kThreads) k_vtx2morton(uint32_t n, uint32_t nu
 template <int kTh>
 __global__ void __launch_bounds__(kTh) k_topology(uint32_t n, const uint32_t* __restrict__ c,
                                                  const uint32_t* __restrict__ idx2obj, uint32_t* bvhnodes,
-                                                 uint32_t* other_end) {
-  pdl_wait();
-  pdl_launch_dependents();
+                                                 uint32_t* other_end, uint32_t* flags, uint32_t* hdr) {
   const uint32_t ib = blockIdx.x * kTh + threadIdx.x;
+  if (flags) {  // idle since before the predecessor, which does not touch them
+    if (ib < n) flags[ib] = 0u;
+    if (ib < kRefitQueueHdr) hdr[ib] = 0u;
+  }
+  pdl_wait();
+  // (no early trigger: the refit's first kernel takes the shared memory of a
+  // whole multiprocessor, and would wait there while branches are still found)
   if (ib >= n - 1) return;
   topology_node(n, Codes32{c}, Objs32{idx2obj}, bvhnodes, ib, other_end);
 }
 
 // A single object: the one-leaf tree [MAX, obj, MAX] (the reference leaves
 // node 0 without children for n == 1).
-__global__ void k_topology_single(const uint32_t* __restrict__ idx2obj, uint32_t* bvhnodes) {
+__global__ void k_topology_single(const uint32_t* __restrict__ idx2obj, uint32_t* bvhnodes, uint32_t* flags,
+                                  uint32_t* hdr) {
+  if (flags && threadIdx.x < kRefitQueueHdr) hdr[threadIdx.x] = 0u;
+  if (threadIdx.x != 0) return;
+  if (flags) flags[0] = 0u;
   bvhnodes[0] = kUMax;
   bvhnodes[1] = idx2obj[0];
   bvhnodes[2] = kUMax;
@@ -402,6 +411,7 @@ __global__ void __launch_bounds__(kThreads) k_refit(uint32_t num_tri, const uint
                                                    const float* __restrict__ vtx2xyz0,
                                                    const float* __restrict__ vtx2xyz1, float* aabb, uint32_t* flags,
                                                    uint32_t* height_out, uint32_t* status, const uint32_t* gate) {
+  pdl_wait();
   // gated (drop-in refit): runs only when the tree was found not to be in
   // Karras leaf order, so that the range queries could not do the call
   if (gate != nullptr && (block_read_hdr(gate, nullptr).x & kRefitPlainClimb) == 0u) return;
@@ -843,6 +853,7 @@ __global__ void __launch_bounds__(kWinThreads) k_refit_seg_win(uint32_t total_tr
                                                               uint32_t* status, const float* __restrict__ tribox,
                                                               const uint32_t* __restrict__ leaf_tri) {
   extern __shared__ __align__(16) unsigned char seg_raw[];
+  pdl_wait();
   Box* tree = reinterpret_cast<Box*>(seg_raw);  // 2 * kRefitWindow boxes
   __shared__ uint32_t s_mesh, s_flag, s_bstar, s_runs;
   const uint32_t wA = blockIdx.x * kRefitWindow;
@@ -1412,23 +1423,32 @@ void launch_vtx2morton(cudaStream_t s, uint32_t n, uint32_t num_dim, const float
 }
 
 void launch_topology(cudaStream_t s, uint32_t n, const uint32_t* idx2morton, const uint32_t* idx2obj,
-                     uint32_t* bvhnodes, uint32_t* other_end, uint32_t threads) {
+                     uint32_t* bvhnodes, uint32_t* other_end, uint32_t threads, uint32_t* flags) {
+  uint32_t* hdr = flags ? flags + refit_queue_offset(n) : nullptr;
   if (n == 1) {
-    k_topology_single<<<1, 1, 0, s>>>(idx2obj, bvhnodes);
+    k_topology_single<<<1, 32, 0, s>>>(idx2obj, bvhnodes, flags, hdr);
     return;
   }
   const uint32_t th = threads == 128 || threads == 512 ? threads : 256u;
-  const uint32_t grid = (n - 1 + th - 1) / th;
-  if (th == 128) launch_pdl(k_topology<128>, dim3(grid), dim3(128), 0, s, n, idx2morton, idx2obj, bvhnodes, other_end);
-  else if (th == 512) launch_pdl(k_topology<512>, dim3(grid), dim3(512), 0, s, n, idx2morton, idx2obj, bvhnodes, other_end);
-  else launch_pdl(k_topology<256>, dim3(grid), dim3(256), 0, s, n, idx2morton, idx2obj, bvhnodes, other_end);
+  const uint32_t grid = (n + th - 1) / th;
+  if (th == 128) launch_pdl(k_topology<128>, dim3(grid), dim3(128), 0, s, n, idx2morton, idx2obj, bvhnodes, other_end,
+                            flags, hdr);
+  else if (th == 512) launch_pdl(k_topology<512>, dim3(grid), dim3(512), 0, s, n, idx2morton, idx2obj, bvhnodes, other_end,
+                            flags, hdr);
+  else launch_pdl(k_topology<256>, dim3(grid), dim3(256), 0, s, n, idx2morton, idx2obj, bvhnodes, other_end,
+                            flags, hdr);
 }
 
-// The kernels after the first of this sequence are launched with launch_pdl
-// and wait (pdl_wait) before touching their predecessor's data, so each is
-// resident when its predecessor ends.  The first kernel triggers nothing
-// early: measured on GB300, letting the range-query kernels' successors in
-// while its last wave runs made the refit slower (2M triangles: 92 -> 115 us).
+// The kernels of this sequence are launched with launch_pdl and wait
+// (pdl_wait) before touching their predecessor's data, so each is resident
+// when its predecessor ends; whoever comes before also zeroes the header (the
+// tree's kernel, a deformation, k_refit_begin), as a memset between kernels
+// costs 4 to 5 us of idle time around it: build, refit and cast of 65 thousand
+// triangles 283 -> 261 us with the cast's memset replaced too, 500 thousand
+// refitted and cast 349 -> 325 us, 64 requests to a server 4596 -> 4456 us.
+// The first kernel triggers nothing early: measured on GB300, letting the
+// range-query kernels' successors in while its last wave runs made the refit
+// slower (2M triangles: 92 -> 115 us).
 void launch_refit_windowed(cudaStream_t s, uint32_t total_tri, const Segments& seg, uint32_t num_vtx_single,
                            const uint32_t* bvhnodes, const uint32_t* other_end, const uint32_t* tri2vtx,
                            const float* vtx2xyz0, const float* vtx2xyz1, float* aabb, uint32_t* flags,
@@ -1475,9 +1495,9 @@ void launch_refit_windowed(cudaStream_t s, uint32_t total_tri, const Segments& s
   float* sseg = const_cast<float*>(v.sseg);
   float* tseg = const_cast<float*>(v.tseg);
   if (seg.tri_off) {
-    k_refit_seg_win<true, false><<<windows, kWinThreads, kSegWinSmem, s>>>(total_tri, seg, num_vtx_single, bvhnodes, other_end, tri2vtx,
-                                                          vtx2xyz0, vtx2xyz1, aabb, queue, flags, wseg, status,
-                                                          nullptr, nullptr);
+    launch_pdl(k_refit_seg_win<true, false>, dim3(windows), dim3(kWinThreads), kSegWinSmem, s, total_tri, seg,
+               num_vtx_single, bvhnodes, other_end, tri2vtx, vtx2xyz0, vtx2xyz1, aabb, queue, flags, wseg, status,
+               static_cast<const float*>(nullptr), nullptr);
     launch_pdl(k_refit_seg_super, dim3(supers), dim3(256), 0, s, total_tri, queue, wseg, sseg, tseg, top_log);
     launch_pdl(k_refit_seg_cross_groups<true, false>, dim3(cross_grid), dim3(256), 0, s, total_tri, seg, other_end, aabb,
                queue, flags, v, cross_groups, status);
@@ -1491,18 +1511,18 @@ void launch_refit_windowed(cudaStream_t s, uint32_t total_tri, const Segments& s
     // run branches are set aside for soups (the meshes with stored triangle
     // boxes), whose clusters make runs of equal codes across windows
     if (tribox) {
-      k_refit_seg_win<false, true><<<windows, kWinThreads, kSegWinSmem, s>>>(total_tri, seg, num_vtx_single, bvhnodes,
-                                                                      other_end, tri2vtx, vtx2xyz0, vtx2xyz1, aabb,
-                                                                      queue, flags, wseg, status, tribox, leaf_tri);
+      launch_pdl(k_refit_seg_win<false, true>, dim3(windows), dim3(kWinThreads), kSegWinSmem, s, total_tri, seg,
+               num_vtx_single, bvhnodes, other_end, tri2vtx, vtx2xyz0, vtx2xyz1, aabb, queue, flags, wseg, status,
+               tribox, leaf_tri);
       launch_pdl(k_refit_seg_super, dim3(supers), dim3(256), 0, s, total_tri, queue, wseg, sseg, tseg, top_log);
       launch_pdl(k_refit_seg_cross_groups<false, true>, dim3(cross_grid), dim3(256), 0, s, total_tri, seg, other_end,
                  aabb, queue, flags, v, cross_groups, status);
       launch_pdl(k_refit_seg_cross_threads<false, true>, dim3(cross_grid1), dim3(256), 0, s, total_tri, seg, other_end,
                  aabb, queue, flags, v, cross_groups, status);
     } else {
-      k_refit_seg_win<false, false><<<windows, kWinThreads, kSegWinSmem, s>>>(total_tri, seg, num_vtx_single, bvhnodes,
-                                                                       other_end, tri2vtx, vtx2xyz0, vtx2xyz1, aabb,
-                                                                       queue, flags, wseg, status, nullptr, leaf_tri);
+      launch_pdl(k_refit_seg_win<false, false>, dim3(windows), dim3(kWinThreads), kSegWinSmem, s, total_tri, seg,
+               num_vtx_single, bvhnodes, other_end, tri2vtx, vtx2xyz0, vtx2xyz1, aabb, queue, flags, wseg, status,
+               static_cast<const float*>(nullptr), leaf_tri);
       launch_pdl(k_refit_seg_super, dim3(supers), dim3(256), 0, s, total_tri, queue, wseg, sseg, tseg, top_log);
       launch_pdl(k_refit_seg_cross_groups<false, false>, dim3(cross_grid), dim3(256), 0, s, total_tri, seg, other_end,
                  aabb, queue, flags, v, cross_groups, status);
@@ -1523,8 +1543,8 @@ void launch_refit(cudaStream_t s, uint32_t num_tri, const uint32_t* bvhnodes, co
   // gated, it usually exits at once: a grid of a few blocks per SM costs
   // less to launch than one thread per leaf
   if (gate != nullptr && grid > 152u * 8u) grid = 152u * 8u;
-  k_refit<<<grid, kThreads, 0, s>>>(num_tri, bvhnodes, tri2vtx, num_vtx, vtx2xyz0, vtx2xyz1, aabb, flags, height_out,
-                                    status, gate);
+  launch_pdl(k_refit, dim3(grid), dim3(kThreads), 0, s, num_tri, bvhnodes, tri2vtx, num_vtx, vtx2xyz0, vtx2xyz1, aabb,
+             flags, height_out, status, gate);
 }
 
 // ------------------------------------------- refit of a tree given as bvhnodes
@@ -1546,6 +1566,12 @@ void launch_refit(cudaStream_t s, uint32_t num_tri, const uint32_t* bvhnodes, co
 // kRefitPlainClimb in the refit header: the range-query kernels exit at once
 // and the parent-pointer climb k_refit does the call.
 constexpr uint32_t kSpineWalk = 64;
+
+// Zeroes the refit header ahead of k_refit_ends, which is resident by then.
+__global__ void k_refit_begin(uint32_t* hdr) {
+  pdl_launch_dependents();
+  if (threadIdx.x < kRefitQueueHdr) hdr[threadIdx.x] = 0u;
+}
 
 __global__ void __launch_bounds__(kThreads) k_refit_ends(uint32_t num_tri, const uint32_t* __restrict__ bn,
                                                          uint32_t* __restrict__ other_end, uint32_t* hdr,
@@ -1590,6 +1616,7 @@ __global__ void __launch_bounds__(kThreads) k_refit_ends(uint32_t num_tri, const
     }
   }
   other_end[i] = bad ? i : (i == lo ? hi : lo);
+  pdl_wait();  // nothing but the header depends on k_refit_begin
   if (bad) atomicOr(hdr + 1, kRefitPlainClimb);
 }
 
@@ -1602,9 +1629,10 @@ void launch_refit_any_tree(cudaStream_t s, uint32_t num_tri, const uint32_t* bvh
     return;
   }
   uint32_t* hdr = flags + refit_queue_offset(num_tri);
-  cudaMemsetAsync(hdr, 0, kRefitQueueHdr * sizeof(uint32_t), s);
   const uint32_t grid = (num_tri + kThreads - 1) / kThreads;
-  k_refit_ends<<<grid, kThreads, 0, s>>>(num_tri, bvhnodes, other_end, hdr, zero_flags ? flags : nullptr);
+  k_refit_begin<<<1, 32, 0, s>>>(hdr);
+  launch_pdl(k_refit_ends, dim3(grid), dim3(kThreads), 0, s, num_tri, bvhnodes, other_end, hdr,
+             zero_flags ? flags : nullptr);
   launch_refit_windowed(s, num_tri, Segments{}, num_vtx, bvhnodes, other_end, tri2vtx, vtx2xyz0, vtx2xyz1, aabb,
                         flags, nullptr, status, nullptr, /*header_ready=*/true);
   launch_refit(s, num_tri, bvhnodes, tri2vtx, num_vtx, vtx2xyz0, vtx2xyz1, aabb, flags, nullptr, status, hdr + 1);

@@ -214,7 +214,6 @@ int build_impl(uint64_t stream_ptr, uint32_t T, const uint32_t* tri2vtx, uint32_
   // the front needs only the header zeroed; the separate kernels also their
   // histograms, tile counters and look-back words
   DM_CUDA(cudaMemsetAsync(base, 0, try_front ? L.sort_hdr : L.sort_hdr + SL.zero_bytes, s));
-  DM_CUDA(cudaMemsetAsync(at<char>(base, L.flags), 0, static_cast<size_t>(T) * 4, s));
   float* transform = at<float>(base, L.transform);
   uint32_t* hist = at<uint32_t>(base, L.sort_hdr + SL.hist);
   uint32_t* counters = at<uint32_t>(base, L.sort_hdr + SL.counters);
@@ -281,11 +280,11 @@ int build_impl(uint64_t stream_ptr, uint32_t T, const uint32_t* tri2vtx, uint32_
     other_end = other_end_out ? other_end_out : (radix10 ? bv : ak);
   }
   if (ev) DM_CUDA(cudaEventRecord(ev[2], s));
-  dm::launch_topology(s, T, ok, ov, bvhnodes, other_end, bt.topo_threads);
+  dm::launch_topology(s, T, ok, ov, bvhnodes, other_end, bt.topo_threads, flags);
   if (ev) DM_CUDA(cudaEventRecord(ev[3], s));
   // the height is only computed on request: it needs the tree-order climb
   dm::launch_refit_windowed(s, T, dm::Segments{1, nullptr, nullptr}, num_vtx, bvhnodes, other_end, tri2vtx, vtx2xyz,
-                            nullptr, aabb, flags, height_out ? height : nullptr, status, tribox, false, ov);
+                            nullptr, aabb, flags, height_out ? height : nullptr, status, tribox, true, ov);
   if (ev) DM_CUDA(cudaEventRecord(ev[4], s));
   if (transform_out) DM_CUDA(cudaMemcpyAsync(transform_out, transform, 64, cudaMemcpyDeviceToDevice, s));
   if (height_out) DM_CUDA(cudaMemcpyAsync(height_out, height, 4, cudaMemcpyDeviceToDevice, s));
@@ -698,7 +697,6 @@ int dm_pix2tri_by_raycast_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t img_h
   if (int e = sc.acquire(scratch, scratch_bytes, dm::cast_scratch_bytes(n, num_tri), s, nullptr)) return e;
   dm::CastScratch cs;
   dm::cast_scratch_carve(sc.ptr, n, num_tri, &cs);
-  DM_CUDA(cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, s));
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb};
   dm::CastOut o{pix2tri, pix2t, nullptr};
   dm::Camera cam;
@@ -731,7 +729,6 @@ int dm_search_bvh3_first_intersection_ray(uint64_t stream_ptr, uint32_t num_ray,
   if (int e = sc.acquire(scratch, scratch_bytes, dm::cast_scratch_bytes(num_ray, num_tri), s, nullptr)) return e;
   dm::CastScratch cs;
   dm::cast_scratch_carve(sc.ptr, num_ray, num_tri, &cs);
-  DM_CUDA(cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, s));
   dm::MeshView m{num_tri, num_vtx, tri2vtx, vtx2xyz, bvhnodes, bvhnode2aabb};
   dm::CastOut o{hit_tri, hit_t, hit_bc};
   dm::launch_cast_rays(s, num_ray, ray_org, ray_dir, m, o, cs, status_ptr());
@@ -953,7 +950,9 @@ int dm_batch_trimesh3_build(uint64_t stream_ptr, uint32_t num_mesh, const uint32
   void* base = sc.ptr;
   uint32_t* status = status_ptr();
   const dm::Segments seg{num_mesh, mesh2tri, mesh2vtx};
-  DM_CUDA(cudaMemsetAsync(at<char>(base, L.flags), 0, size_t{4} * total_tri, s));
+  // the refit's arrival counters and, next to them, its header
+  DM_CUDA(cudaMemsetAsync(at<char>(base, L.flags), 0,
+                          4 * (dm::refit_queue_offset(total_tri) + dm::kRefitQueueHdr), s));
   if (max_tri_per_mesh <= dm::kSegMaxTri && dm::get_tuning().batch_path == 0) {
     // every mesh sorted and linked on chip (the lists reuse the key buffer)
     uint32_t* seg_counters = at<uint32_t>(base, L.counters) + 8;
@@ -962,7 +961,7 @@ int dm_batch_trimesh3_build(uint64_t stream_ptr, uint32_t num_mesh, const uint32
                                    at<uint32_t>(base, L.keys_a), seg_counters, status) != 0)
       return fail(DM_ERR_CUDA, "fused batch build launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     dm::launch_refit_windowed(s, total_tri, seg, 0, bvhnodes, at<uint32_t>(base, L.other), tri2vtx, vtx2xyz, nullptr,
-                              bvhnode2aabb, at<uint32_t>(base, L.flags), heights, status);
+                              bvhnode2aabb, at<uint32_t>(base, L.flags), heights, status, nullptr, /*header_ready=*/true);
     DM_CUDA(cudaGetLastError());
     return DM_OK;
   }
@@ -989,7 +988,7 @@ int dm_batch_trimesh3_build(uint64_t stream_ptr, uint32_t num_mesh, const uint32
   }
   dm::launch_batch_topology(s, total_tri, seg, ks, vs, bvhnodes, at<uint32_t>(base, L.other));
   dm::launch_refit_windowed(s, total_tri, seg, 0, bvhnodes, at<uint32_t>(base, L.other), tri2vtx, vtx2xyz, nullptr,
-                            bvhnode2aabb, at<uint32_t>(base, L.flags), heights, status);
+                            bvhnode2aabb, at<uint32_t>(base, L.flags), heights, status, nullptr, /*header_ready=*/true);
   DM_CUDA(cudaGetLastError());
   return DM_OK;
 }
@@ -1018,7 +1017,6 @@ int dm_batch_pix2tri_by_raycast(uint64_t stream_ptr, uint32_t num_mesh, const ui
   if (int e = sc.acquire(scratch, scratch_bytes, dm::cast_scratch_bytes(n, max_tri_per_mesh), s, nullptr)) return e;
   dm::CastScratch cs;
   dm::cast_scratch_carve(sc.ptr, n, max_tri_per_mesh, &cs);
-  DM_CUDA(cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, s));
   dm::CastOut o{pix2tri, pix2t, nullptr};
   dm::launch_batch_cast_pixels(s, dm::Segments{num_mesh, mesh2tri, mesh2vtx}, max_tri_per_mesh, tri2vtx, vtx2xyz,
                                bvhnodes, bvhnode2aabb, img_w, img_h, transforms_ndc2world, o, cs, status_ptr());

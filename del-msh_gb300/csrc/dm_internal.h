@@ -48,9 +48,13 @@ void launch_vtx2morton(cudaStream_t s, uint32_t n, uint32_t num_dim, const float
 
 // bvhnodes_morton.rs:10-50 / bvhnodes_morton.cu:29-72.  other_end (optional,
 // u32[n-1]): for each branch the end of its leaf range that is not its own
-// index (a branch index is always one end of its range).
+// index (a branch index is always one end of its range).  flags (optional,
+// u32[refit_flags_words(n)]): the arrival counters and the refit header in it
+// are zeroed on the way, so that launch_refit_windowed may follow with
+// header_ready.
 void launch_topology(cudaStream_t s, uint32_t n, const uint32_t* idx2morton, const uint32_t* idx2obj,
-                     uint32_t* bvhnodes, uint32_t* other_end = nullptr, uint32_t threads = 256);
+                     uint32_t* bvhnodes, uint32_t* other_end = nullptr, uint32_t threads = 256,
+                     uint32_t* flags = nullptr);
 
 // Vertex indices >= num_vtx are replaced by 0 and raise kStatusBadIndex.
 // Bottom-up refit (bvhnode2aabb.cu:7-65 semantics, values of
@@ -305,7 +309,7 @@ struct CastOut {
 constexpr size_t kCastCounterBytes = 32;
 
 struct CastScratch {
-  uint32_t* counters;  // kCastCounterBytes, zero on entry (see cast_job)
+  uint32_t* counters;  // kCastCounterBytes (see cast_job)
   uint32_t* list1;     // num_ray words
   uint32_t* list2;     // num_ray words
   void* pool;          // >= 16 * max(num_tri, 4096) bytes

@@ -435,6 +435,7 @@ __global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_pers
                                                                                  Parked parked) {
   __shared__ float smem[64];
   job.prepare(smem);
+  pdl_wait();  // k_cast_begin
   __syncthreads();
   constexpr uint32_t kAll = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31;
@@ -1217,6 +1218,14 @@ inline uint32_t park_steps(uint32_t num_work) {
 // it takes: warps are filled and nothing is parked, as helpers also search
 // subtrees that turn out not to be needed.  64 requests in flight at once took
 // 4.65 ms so and 5.01 ms with parking.
+// Zeroes a cast's counters.  A kernel instead of a copy-engine memset, so that
+// the persistent cast's blocks are resident when it ends.
+static __global__ void k_cast_begin(uint32_t* counters) {
+  pdl_wait();
+  pdl_launch_dependents();
+  if (threadIdx.x < kCastCounterBytes / sizeof(uint32_t)) counters[threadIdx.x] = 0u;
+}
+
 template <typename Job, int kThreads, int kStack>
 inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, bool busy,
                          uint32_t* status) {
@@ -1259,14 +1268,15 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   a.max_tri = max_tri;
   a.long_steps = t.cast_long_steps;
   a.status = status;
-  k_cast_persistent<Job, kThreads, kStack><<<grid, kThreads, 0, s>>>(job, sc.counters, sc.list1, sc.counters + 1,
-                                                                     status, mins, a.parked);
+  launch_pdl(k_cast_begin, dim3(1), dim3(32), 0, s, sc.counters);
+  launch_pdl(k_cast_persistent<Job, kThreads, kStack>, dim3(grid), dim3(kThreads), 0, s, job, sc.counters, sc.list1,
+             sc.counters + 1, status, mins, a.parked);
   launch_pdl(k_cast_tail<Job, kStack>, dim3(152 * 4), dim3(kTeamThreads), 0, s, job, a);
 }
 
 // The tiered cast of every work index of `job`: the persistent cast, then one
 // kernel for the rays it hands over (k_cast_tail).  sc.counters
-// (kCastCounterBytes) must be zero on entry: [0] rays taken, [1] rays for the
+// (kCastCounterBytes) are zeroed first: [0] rays taken, [1] rays for the
 // team tier (list1), [2], [3] rays for the two deep casts (list2, list1 again),
 // [4] rays taken by the team tier, [5] rays parked, [6] parked rays taken, [7]
 // blocks done.  The first tier's block size and on-chip stack depth come from

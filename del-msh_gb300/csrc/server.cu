@@ -65,10 +65,13 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   return x;
 }
 
-// v = rest + amp * sin(phase_v + frame + axis)
+// v = rest + amp * sin(phase_v + frame + axis); also zeroes the header of the
+// refit that follows
 __global__ void k_deform(uint32_t num_vtx, const float* __restrict__ rest, float* __restrict__ out, uint32_t seed,
-                         uint32_t frame, float amp) {
+                         uint32_t frame, float amp, uint32_t* refit_hdr) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0)
+    for (uint32_t k = 0; k < kRefitQueueHdr; ++k) refit_hdr[k] = 0u;
   if (i >= num_vtx) return;
   const float phase = static_cast<float>(hash32(seed ^ (i * 0x9E3779B9u))) * (6.2831853f / 4294967296.0f);
 #pragma unroll
@@ -211,10 +214,11 @@ int prepare_mesh(cudaStream_t st, const HostMesh& hm, DevMesh& m, uint32_t kind,
     if (frame == 0) {
       if (cudaMemcpyAsync(m.vtx, m.rest, 12ull * hm.V, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return DM_ERR_CUDA;
     } else {
-      k_deform<<<(hm.V + 255) / 256, 256, 0, st>>>(hm.V, m.rest, m.vtx, hm.seed, frame, amp);
+      k_deform<<<(hm.V + 255) / 256, 256, 0, st>>>(hm.V, m.rest, m.vtx, hm.seed, frame, amp,
+                                                     m.flags + refit_queue_offset(hm.T));
     }
     launch_refit_windowed(st, hm.T, Segments{1, nullptr, nullptr}, hm.V, m.bvh, m.other, m.tri, m.vtx, nullptr,
-                          m.aabb, m.flags, nullptr, device_status_word());
+                          m.aabb, m.flags, nullptr, device_status_word(), nullptr, /*header_ready=*/frame != 0);
     m.frame = frame;
     m.amp = amp;
     if (counters) counters->refits++;
@@ -230,7 +234,6 @@ int cast_request(cudaStream_t st, const HostMesh& hm, const DevMesh& m, const dm
   CastScratch cs;
   const uint32_t n = (r.kind == DM_REQ_CAST_RAYS) ? r.num_ray : r.img_w * r.img_h;
   cast_scratch_carve(sl.cast_scratch, n, hm.T, &cs);
-  if (cudaMemsetAsync(cs.counters, 0, dm::kCastCounterBytes, st) != cudaSuccess) return DM_ERR_CUDA;
   CastOut o{sl.d_hit, sl.d_t, nullptr};
   if (r.kind == DM_REQ_CAST_RAYS) {
     float* org = sl.d_rays;
