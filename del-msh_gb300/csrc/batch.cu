@@ -668,6 +668,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_seg_classify(Segments seg, u
 
 struct BatchJob {
   static constexpr uint32_t kRefillHalves = 3;
+  static constexpr int kCastRegs = 56;
   uint32_t num_work;
   Segments seg;
   const uint32_t* tri2vtx;

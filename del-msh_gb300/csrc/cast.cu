@@ -14,6 +14,7 @@ namespace {
 
 struct SingleJob {
   static constexpr uint32_t kRefillHalves = 2;
+  static constexpr int kCastRegs = 64;
   uint32_t num_work;
   MeshView m;
   uint32_t img_w, img_h, tiles_x, tile_w, tile_h;  // pixel mode

@@ -395,6 +395,7 @@ constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 //                                                   m becomes that of lane `from` (all lanes call it)
 //   __device__ void write(uint32_t out, const MeshView& m, const Ray& r, const Hit& h) const;
 //   kRefillHalves                                   halves of cast_refill_min at which a warp takes rays
+//   kCastRegs                                       registers a thread of the persistent cast
 
 // Thresholds of the phased loop: a phase runs when at least this many lanes
 // of the warp wait for it, or when nothing else can run.
@@ -423,12 +424,16 @@ struct Parked {
 // thresholds.  Rays overflowing the on-chip stack, and rays past mins.long_steps
 // node entries at a long chain once the warp's work is exhausted, go to ovf_list
 // (their work index) for the team tier.  kThreads threads per block and kStack
-// on-chip frames per ray are tuning choices (Tuning); the register bound (64
-// registers) keeps 2048 resident threads per SM.  The loop after the work has run
+// on-chip frames per ray are tuning choices (Tuning).  The register bound is the
+// job's: the cast waits for loads most of all (a third of its stalls), and 56
+// registers keep 36 warps resident where 64 keep 32.  For the batch that pays,
+// 64 / 56 / 48 registers: 1220 / 1173 / 1195 us; one mesh's cast spills more and
+// is also held by single rays: 2M triangles at 1920 x 1080 431 / 440 / 446 us,
+// 16,384 rays 136 / 143 / 144 us.  The loop after the work has run
 // out is a second copy of the phases: with one loop for both, the parking code
 // cost the first one 100 bytes of spills (batched cast 1.26 -> 1.48 ms).
 template <typename Job, int kThreads, int kStack>
-__global__ void __launch_bounds__(kThreads, 65536 / (64 * kThreads)) k_cast_persistent(Job job, uint32_t* work_counter,
+__global__ void __launch_bounds__(kThreads, 65536 / (Job::kCastRegs * kThreads)) k_cast_persistent(Job job, uint32_t* work_counter,
                                                                                  uint32_t* ovf_list,
                                                                                  uint32_t* ovf_count,
                                                                                  uint32_t* status, PhaseMins mins,
