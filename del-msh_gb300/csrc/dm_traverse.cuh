@@ -1112,9 +1112,16 @@ struct TailArgs {
 // A team is a whole block while the rays are few, kTeamRays per block or
 // fewer: then the longest ray sets the kernel's end.  With more, their number
 // does, and each warp takes rays of its own.
+// Blocks a multiprocessor of the tail kernel: 6 (80 registers, 76 bytes of spills)
+// let the split tier of large images hold more rays at once than 4 (124
+// registers) and cost the others nothing; 2M triangles at 1920 x 1080 with 4, 5,
+// 6, 8: 431, 432, 407, 416 us, 16,384 rays 135, 130, 132, 138 us, 512 x 512 of
+// 502 thousand triangles 212, 213, 213, 220 us, a soup's rays 657, 642, 655,
+// 709 us.
+constexpr uint32_t kTailBlocks = 6;
 constexpr uint32_t kTeamRays = 8;
 template <typename Job, int kStack>
-__global__ void __launch_bounds__(kTeamThreads, 4) k_cast_tail(Job job, TailArgs a) {
+__global__ void __launch_bounds__(kTeamThreads, kTailBlocks) k_cast_tail(Job job, TailArgs a) {
   __shared__ float smem[64];
   __shared__ FoldShared sh[kTeamWarps];
   __shared__ uint2 sh_deal[kTeamThreads];
@@ -1276,7 +1283,7 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   launch_pdl(k_cast_begin, dim3(1), dim3(32), 0, s, sc.counters);
   launch_pdl(k_cast_persistent<Job, kThreads, kStack>, dim3(grid), dim3(kThreads), 0, s, job, sc.counters, sc.list1,
              sc.counters + 1, status, mins, a.parked);
-  launch_pdl(k_cast_tail<Job, kStack>, dim3(152 * 4), dim3(kTeamThreads), 0, s, job, a);
+  launch_pdl(k_cast_tail<Job, kStack>, dim3(152 * kTailBlocks), dim3(kTeamThreads), 0, s, job, a);
 }
 
 // The tiered cast of every work index of `job`: the persistent cast, then one
