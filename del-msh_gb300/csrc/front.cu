@@ -11,7 +11,9 @@
 // a 16 us pass.  Here the tiles publish their digit counts, a grid barrier
 // follows, one warp per digit scans that digit's counts over the tiles
 // (exclusive prefix per tile, and the digit's total), a second barrier
-// follows, and every tile then knows its output offsets at once.  The same
+// follows, and every tile then knows its output offsets at once (few tiles do
+// without the scan: kDirectTiles).  What bounds the kernel at small sizes is the
+// barriers, about 2 us each, and the chains between them.  The same
 // barriers let the centroids stay in shared memory between the AABB pass and
 // the Morton codes, and the codes stay in registers into the first pass, so
 // neither is written to memory and read back.
@@ -38,6 +40,18 @@ namespace {
 constexpr int kFThreads = 512;
 constexpr int kFWarps = kFThreads / 32;
 constexpr int kFRadix = 256;
+// Up to this many tiles, every tile adds up the counts of all tiles by itself
+// (half of the tiles per thread, 8 rows in flight) instead of waiting for the
+// column scan and a second barrier.  Builds in us by scan / by sums: 3 tiles
+// 80 / 56, 64 tiles 76 / 68 (64 tiles of 2048 keys: 64), 123 tiles of 4096 keys
+// 93 / 96, 256 tiles 136 / 147.
+constexpr uint32_t kDirectTiles = 96;
+// Up to this many tiles a tile has 2048 keys, half of the next larger: its
+// ranking and gathers are chains of that length, and the multiprocessors are
+// not short of blocks.  Builds in us with 4096 / 2048 keys: 5,000 triangles
+// 56 / 49, 65,522 triangles 68 / 62, 262,088 triangles 79 / 74; at 500,000 (245
+// tiles of 2048) 96 / 108.
+constexpr uint32_t kSmallTiles = 152;
 
 struct FMinMax {
   float lo[3], hi[3];
@@ -77,7 +91,8 @@ struct FrontArgs {
   uint32_t* tri2morton;  // codes in triangle order, or nullptr
   uint32_t *ka, *va, *kb, *vb;       // ping-pong buffers, num_tri words each
   uint32_t *out_keys, *out_vals;     // sorted codes and triangle indices (not ka / va)
-  uint32_t* counts;      // [256][grid]: per-tile digit counts, then exclusive prefixes
+  uint32_t* counts;      // [256][grid]: per-tile digit counts, then exclusive prefixes;
+                         // [grid][256] counts up to kDirectTiles
   uint32_t* totals;      // [256]: per-digit totals of the current pass
   uint32_t* bar;         // grid-barrier counter, zero at launch
   uint32_t* status;
@@ -357,6 +372,7 @@ __global__ void __launch_bounds__(kFThreads, 2) k_build_front(FrontArgs a) {
 
   // ---- the four stable 8-bit passes: computed -> A -> B -> A -> out
   const uint32_t lt_mask = (1u << lane) - 1u;
+  const bool direct = nt <= kDirectTiles;
 #pragma unroll 1
   for (int p = 0; p < 4; ++p) {
     const uint32_t shift = 8u * p;
@@ -412,7 +428,7 @@ __global__ void __launch_bounds__(kFThreads, 2) k_build_front(FrontArgs a) {
         S.u.s.whist[w][tid] = static_cast<uint16_t>(cnt);  // <= kTile - 1
         cnt += c;
       }
-      a.counts[static_cast<size_t>(tid) * nt + tile] = cnt;
+      a.counts[direct ? static_cast<size_t>(tile) * kFRadix + tid : static_cast<size_t>(tid) * nt + tile] = cnt;
     }
     const uint32_t ts = block_exclusive_scan512(cnt, S.scan);  // has __syncthreads
     if (tid < kFRadix) S.tstart[tid] = ts;
@@ -440,40 +456,69 @@ __global__ void __launch_bounds__(kFThreads, 2) k_build_front(FrontArgs a) {
     }
     grid_barrier(a.bar, epoch, a.status, a.spin_limit);  // every tile's counts are published
 
-    // one warp per digit: exclusive prefix of the digit's counts over the
-    // tiles (in place) and the digit's total; lane l holds tiles l, l+32, ...
-    // of a chunk of 256 tiles, loaded together
-    for (uint32_t d = tile * kFWarps + warp; d < kFRadix; d += nt * kFWarps) {
-      uint32_t* col = a.counts + static_cast<size_t>(d) * nt;
-      uint32_t carry = 0;
-      for (uint32_t r0 = 0; r0 < nt; r0 += 256) {
+    uint32_t tot = 0, pre = 0;  // tid < 256: the digit's total, and its keys in the tiles before this one
+    if (direct) {
+      const uint32_t d = static_cast<uint32_t>(tid) % kFRadix, half = static_cast<uint32_t>(tid) / kFRadix;
+      const uint32_t mid = (nt + 1) / 2, t1 = half ? nt : mid;
+      const uint32_t* row = a.counts + d;
+      for (uint32_t t0 = half ? mid : 0u; t0 < t1; t0 += 8) {
         uint32_t v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t t = r0 + 32u * i + lane;
-          v[i] = t < nt ? __ldcg(col + t) : 0u;
-        }
+        for (int i = 0; i < 8; ++i) v[i] = t0 + i < t1 ? __ldcg(row + static_cast<size_t>(t0 + i) * kFRadix) : 0u;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          uint32_t x = v[i];
-#pragma unroll
-          for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-          }
-          const uint32_t t = r0 + 32u * i + lane;
-          if (t < nt) col[t] = carry + x - v[i];
-          carry += __shfl_sync(0xffffffffu, x, 31);
+          tot += v[i];
+          if (t0 + i < tile) pre += v[i];
         }
       }
-      if (lane == 0) a.totals[d] = carry;
+      uint32_t* other = &S.u.s.match[0][0];  // idle until the next pass clears it
+      if (half) {
+        other[d] = tot;
+        other[kFRadix + d] = pre;
+      }
+      __syncthreads();
+      if (!half) {
+        tot += other[d];
+        pre += other[kFRadix + d];
+      }
+    } else {
+      // one warp per digit: exclusive prefix of the digit's counts over the
+      // tiles (in place) and the digit's total; lane l holds tiles l, l+32, ...
+      // of a chunk of 256 tiles, loaded together
+      for (uint32_t d = tile * kFWarps + warp; d < kFRadix; d += nt * kFWarps) {
+        uint32_t* col = a.counts + static_cast<size_t>(d) * nt;
+        uint32_t carry = 0;
+        for (uint32_t r0 = 0; r0 < nt; r0 += 256) {
+          uint32_t v[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t t = r0 + 32u * i + lane;
+            v[i] = t < nt ? __ldcg(col + t) : 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            uint32_t x = v[i];
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+              const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+              if (lane >= off) x += y;
+            }
+            const uint32_t t = r0 + 32u * i + lane;
+            if (t < nt) col[t] = carry + x - v[i];
+            carry += __shfl_sync(0xffffffffu, x, 31);
+          }
+        }
+        if (lane == 0) a.totals[d] = carry;
+      }
+      grid_barrier(a.bar, epoch, a.status, a.spin_limit);  // prefixes and totals are complete
+      if (tid < kFRadix) {
+        tot = __ldcg(a.totals + tid);
+        pre = __ldcg(a.counts + static_cast<size_t>(tid) * nt + tile);
+      }
     }
-    grid_barrier(a.bar, epoch, a.status, a.spin_limit);  // prefixes and totals are complete
 
-    const uint32_t tot = tid < kFRadix ? __ldcg(a.totals + tid) : 0u;
-    const uint32_t gb = block_exclusive_scan512(tot, S.scan);  // has __syncthreads
-    if (tid < kFRadix)
-      S.offs[tid] = gb + __ldcg(a.counts + static_cast<size_t>(tid) * nt + tile) - S.tstart[tid];  // mod 2^32
+    const uint32_t gb = block_exclusive_scan512(tid < kFRadix ? tot : 0u, S.scan);  // has __syncthreads
+    if (tid < kFRadix) S.offs[tid] = gb + pre - S.tstart[tid];  // mod 2^32
     __syncthreads();
     for (uint32_t i = tid; i < tile_n; i += kFThreads) {
       const uint32_t key = S.u.s.keys[i];
@@ -500,7 +545,7 @@ FrontVariant front_variant() {
 
 // Blocks of `v` that fit on the device at once (per device, looked up once).
 uint32_t front_capacity(const FrontVariant& v, int slot) {
-  static uint32_t cap[64][6] = {};
+  static uint32_t cap[64][8] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   if (cap[dev][slot] == 0) {
@@ -523,7 +568,7 @@ uint32_t front_capacity(const FrontVariant& v, int slot) {
 
 uint32_t front_max_tri() {
   const FrontVariant v = front_variant<16, false>();
-  const uint64_t c = front_capacity(v, 4);
+  const uint64_t c = front_capacity(v, 6);
   const uint64_t m = c * kFThreads * 16;
   return m > 0xFFFFFFFFull ? 0xFFFFFFFFu : static_cast<uint32_t>(m);
 }
@@ -535,15 +580,16 @@ bool launch_build_front(cudaStream_t s, uint32_t num_tri, const uint32_t* tri2vt
                         uint32_t* totals, uint32_t* bar, uint32_t* status) {
   if (num_tri < 2) return false;
   const bool box = tribox != nullptr;
-  const FrontVariant vs[3] = {box ? front_variant<8, true>() : front_variant<8, false>(),
+  const FrontVariant vs[4] = {box ? front_variant<4, true>() : front_variant<4, false>(),
+                              box ? front_variant<8, true>() : front_variant<8, false>(),
                               box ? front_variant<12, true>() : front_variant<12, false>(),
                               box ? front_variant<16, true>() : front_variant<16, false>()};
-  for (int k = 0; k < 3; ++k) {
+  for (int k = 0; k < 4; ++k) {
     const FrontVariant& v = vs[k];
     const uint32_t tile = static_cast<uint32_t>(kFThreads * v.kpt);
     const uint32_t grid = (num_tri + tile - 1) / tile;
     const uint32_t cap = front_capacity(v, 2 * k + (box ? 1 : 0));
-    if (grid > cap || grid > max_partials) continue;
+    if (grid > cap || grid > max_partials || (k == 0 && grid > kSmallTiles)) continue;
     FrontArgs args{num_tri, num_vtx, tri2vtx, vtx2xyz, tribox, partials, transform_out, aabb_out, tri2morton,
                    ka, va, kb, vb, out_keys, out_vals, counts, totals, bar, status, get_wait_limit()};
     void* params[] = {&args};

@@ -8,8 +8,10 @@
 // microsecond or two.  One block does the same work without leaving its SM.
 // Back-to-back builds (displaced tori), us:
 //   triangles      18    60   242   968  1250  1984  3960
-//   many kernels   91    91    89   101   105   109   111
-//   one block     6.2   6.5   8.2    17    27    30    58
+//   many kernels   36    36    37    41    44    48    53
+//   one block     6.2   6.5   7.9    16    26    29    56
+// (From 2,700 triangles on the two are within 3 us, where one launch instead of
+// nine still decides: each costs a caller without a captured graph 2 us or more.)
 // What bounds it from there on is one SM's instruction issue, in the sort first;
 // at 4,096 triangles (two heaps of boxes, 213 KB) the shared memory is full too.
 //
