@@ -1211,17 +1211,24 @@ inline int persistent_grid() {
 }
 
 // Node entries after which a ray is parked: kParkSteps for up to kParkRays rays,
-// kParkMore more for each doubling.  Parked too early, rays crowd the split
-// tier; too late, they hold the persistent cast.  Casts in us by threshold:
+// kParkMore more for each of the first kParkDoublings doublings.  Parked too early,
+// rays crowd the split tier; too late, they hold the persistent cast.  Casts in us
+// by threshold:
 //   16,384 rays on a jittered sphere    24: 136   40: 142   64: 160   96: 185   never: 194
 //   641 x 479 on a torus                40: 177   64: 156   80: 159  112: 184   never: 193
 //   512 x 512 on a deformed torus       40: 286   64: 251   80: 235  112: 240   never: 324
-//   1920 x 1080 on a 2M torus           64: 513   96: 446  112: 419  144: 426   never: 603
-constexpr uint32_t kParkSteps = 24, kParkRays = 16384, kParkMore = 14;
+// and, means over six 2M tori (never: before there was parking)
+//   1280 x 720                          94: 385  140: 415  180: 452  220: 473   never: 537
+//   1920 x 1080                         80: 532   94: 520  108: 529  150: 529   never: 629
+//   2560 x 1440                         88: 690   94: 697  122: 700  150: 704   never: 765
+//   3840 x 2160                         88: 1194  94: 1191 108: 1190 150: 1209  never: 1252
+// Where no ray goes on for long, the tail's fixed time is not won back: on the
+// smoothest two of the six, 1920 x 1080 takes 485 and 497 us against 465 and 467.
+constexpr uint32_t kParkSteps = 24, kParkRays = 16384, kParkMore = 14, kParkDoublings = 5;
 
 inline uint32_t park_steps(uint32_t num_work) {
   uint32_t doublings = 0;
-  for (uint32_t n = num_work; n >= 2 * kParkRays; n >>= 1) ++doublings;
+  for (uint32_t n = num_work; n >= 2 * kParkRays && doublings < kParkDoublings; n >>= 1) ++doublings;
   return kParkSteps + kParkMore * doublings;
 }
 
