@@ -390,7 +390,8 @@ void launch_octree_aggregate(cudaStream_t s, uint32_t num_idx, uint32_t num_vdim
 // Self-intersecting triangle pairs through the BVH: pairs u32[capacity][2],
 // segments f32[capacity][6]; *count (zero on entry) receives the number
 // found, which may exceed capacity (then only capacity are written).
-// Synchronizes the stream once per round (to size the next).  scratch:
+// Synchronizes the stream after every fourth round (to see whether there is
+// another).  scratch:
 // self_intersection_scratch_bytes(num_tri).  Returns 0, or -1 on a CUDA error.
 size_t self_intersection_scratch_bytes(uint32_t num_tri);
 int launch_self_intersection(cudaStream_t s, const MeshView& m, uint32_t capacity, uint32_t* pairs, float* segments,

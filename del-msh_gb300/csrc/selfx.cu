@@ -204,7 +204,8 @@ __device__ __forceinline__ void report_pair(const MeshView& m, uint32_t a0, uint
 // threads: 4.24 ms for two crossing tori of 260,084 triangles in all, against
 // 0.33 ms for the four rounds here.
 constexpr uint32_t kWarpsPerBlock = kThreads / 32;
-constexpr uint32_t kPairStack = 704;   // node pairs on a warp's stack
+constexpr uint32_t kPairStack = 784;   // node pairs on a warp's stack (the most that leaves 8 blocks per SM)
+constexpr uint32_t kWideStack = 592;   // of them while pairs are popped several at a time
 constexpr uint32_t kLeafBuffer = 64;   // leaf pairs waiting for their test
 // Every so many steps a warp looks whether the round's start pairs are all
 // given out; if so warps are running idle, and it hands its own pairs to the
@@ -213,7 +214,16 @@ constexpr uint32_t kLeafBuffer = 64;   // leaf pairs waiting for their test
 // side took 1.49, 1.18, 1.03 and 1.08 ms for 8, 16, 32 and 64 steps.
 constexpr uint32_t kRoundSteps = 32;
 
-constexpr uint32_t kAloneLooks = 2048, kAloneMost = 1u << 17;  // looks of a search that nothing ends
+constexpr uint32_t kAloneLooks = 2048;  // looks of a search that nothing ends
+
+// A warp whose next list is full goes on alone, and must not run out of stack:
+// popping 32 pairs whose boxes all overlap pushes up to 128.  From then on it pops
+// a twelfth of what is left below kWideStack, 1 at the least, which settles at
+// some 10 pairs a step where everything overlaps everything (a host model of the
+// stack; a third of what is left settles at 2).  The 192 entries above kWideStack
+// hold 64 levels of a search by single pairs, each of which leaves three behind.
+constexpr uint32_t kNarrowPart = 12;
+static_assert((kPairStack - kWideStack) / 3 >= 64, "levels of a search by single pairs");
 
 // A round's start pairs are `start[0 .. *num_start)`, or without a list the
 // children (left(n), right(n)) of every branch n.
@@ -224,40 +234,55 @@ struct RoundList {
   uint2* next;         // the next round's list
   uint32_t* num_next;
   uint32_t next_cap;
+  // pairs popped over all rounds, and how many there can be: a tree has each pair
+  // of nodes once, so a search beyond that is one without an end (a cycle)
+  unsigned long long* popped;
+  unsigned long long most;
 };
 
-// Moves the `k` bottom pairs of the stack to the next round's list if they all
-// fit there.
-__device__ __forceinline__ bool hand_over(const RoundList& rl, uint2* stack, uint32_t& sp, uint32_t k, uint32_t lane) {
-  uint32_t at = 0, ok = 0;
+// Moves the `k` bottom pairs of the stack, those with the most below them, to the
+// next round's list: all of them while the list is less than half full, else none,
+// or with `some` a small part of what is free, so that every warp that is still
+// busy at the end of a round finds room for its largest pairs, look after look
+// (131,072 triangles whose boxes all overlap, 8.6e9 pairs of leaves: 14.8 s with
+// whole stacks or nothing up to the end of the list, as the last warps of a round
+// then search on alone, and 0.43 s so).  Returns how many.
+__device__ __forceinline__ uint32_t hand_over(const RoundList& rl, uint2* stack, uint32_t& sp, uint32_t k, bool some,
+                                              uint32_t lane) {
+  uint32_t at = 0, got = 0;
   if (lane == 0) {
     // a reservation that would pass the end is refused by compare-and-swap, so
     // that the list has no unwritten holes (a bounded number of attempts)
+    const uint32_t half = rl.next_cap / 2;
     uint32_t cur = *reinterpret_cast<volatile uint32_t*>(rl.num_next);
-    for (int attempt = 0; attempt < 64 && cur <= rl.next_cap && k <= rl.next_cap - cur; ++attempt) {
-      const uint32_t seen = atomicCAS(rl.num_next, cur, cur + k);
+    for (int attempt = 0; attempt < 64; ++attempt) {
+      uint32_t n = k;
+      if (cur > half || k > half - cur)
+        n = some ? min(min(k, (rl.next_cap - cur + 65535u) / 65536u), rl.next_cap - cur) : 0u;
+      if (n == 0) break;
+      const uint32_t seen = atomicCAS(rl.num_next, cur, cur + n);
       if (seen == cur) {
         at = cur;
-        ok = 1;
+        got = n;
         break;
       }
       cur = seen;
     }
   }
   at = __shfl_sync(0xffffffffu, at, 0);
-  ok = __shfl_sync(0xffffffffu, ok, 0);
-  if (!ok) return false;
-  for (uint32_t q = lane; q < k; q += 32) rl.next[at + q] = stack[q];
+  got = __shfl_sync(0xffffffffu, got, 0);
+  if (got == 0) return 0;
+  for (uint32_t q = lane; q < got; q += 32) rl.next[at + q] = stack[q];
   __syncwarp();
   // the rest moves down, 32 pairs at a time (each read before it is overwritten)
-  for (uint32_t q = k; q < sp; q += 32) {
+  for (uint32_t q = got; q < sp; q += 32) {
     const uint2 v = q + lane < sp ? stack[q + lane] : make_uint2(0, 0);
     __syncwarp();
-    if (q + lane < sp) stack[q + lane - k] = v;
+    if (q + lane < sp) stack[q + lane - got] = v;
     __syncwarp();
   }
-  sp -= k;
-  return true;
+  sp -= got;
+  return got;
 }
 
 template <bool kVec>
@@ -275,8 +300,9 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
   // start pairs are dealt out a few at a time (8 against 32: 0.95 against 1.03 ms,
   // as fewer warps end with much left), and one by one when there are few
   const uint32_t chunk = min(8u, max(1u, num_start / (gridDim.x * kWarpsPerBlock)));
-  uint32_t sp = 0, nleaf = 0, steps = 0, alone = 0;
-  bool more = num_start > 0, bad = false;
+  uint32_t sp = 0, nleaf = 0, steps = 0, alone = 0, popped = 0;
+  bool bad = __any_sync(kAll, *reinterpret_cast<volatile unsigned long long*>(rl.popped) > rl.most);
+  bool more = num_start > 0 && !bad, full = false;  // full: the next list had no room
   for (;;) {
     bool live = false;  // this lane holds a pair of branches, or of a branch and a leaf
     uint32_t a = 0, b = 0, a0 = 0, a1 = 0, b0 = 0, b1 = 0;
@@ -317,27 +343,31 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
       // split; a search of this length without an end (a tree with a cycle,
       // for which the rounds are the bound) is handed over all the same
       uint32_t taken = 0;
-      if (lane == 0) taken = *reinterpret_cast<volatile uint32_t*>(rl.take);
-      taken = __shfl_sync(kAll, taken, 0);
-      if ((taken >= num_start || alone >= kAloneLooks) && hand_over(rl, stack, sp, sp, lane)) {
-        alone = 0;
-        continue;
+      bool endless = false;
+      if (lane == 0) {
+        taken = *reinterpret_cast<volatile uint32_t*>(rl.take);
+        endless = atomicAdd(rl.popped, static_cast<unsigned long long>(popped)) + popped > rl.most;
       }
-      if (++alone > kAloneMost) {  // no room in the list, and no end
-        if (lane == 0) raise_status(status, kStatusStackOverflow);
+      popped = 0;
+      if (__any_sync(kAll, endless)) {
+        bad = true;
         break;
       }
+      taken = __shfl_sync(kAll, taken, 0);
+      if ((taken >= num_start || alone >= kAloneLooks) && hand_over(rl, stack, sp, sp, true, lane) != 0) {
+        alone = 0;
+        full = full && sp + 96 > kWideStack;
+        continue;
+      }
+      ++alone;
     }
     ++steps;
-    // a popped pair leaves room for at most four: fewer are popped while the
-    // stack is nearly full, after handing its older half on if that fits
-    if (sp + 96 > kPairStack) hand_over(rl, stack, sp, sp / 2, lane);
-    const uint32_t room = (kPairStack - sp) / 3;
-    if (room == 0) {
-      if (lane == 0) raise_status(status, kStatusStackOverflow);
-      break;
-    }
-    const uint32_t k = min(min(32u, sp), room);
+    // a popped pair leaves room for at most four, so 32 are popped only while the
+    // stack takes their children; before that its older half is handed on
+    if (sp + 96 > kWideStack && !full) full = hand_over(rl, stack, sp, sp / 2, false, lane) == 0;
+    const uint32_t narrow = sp < kWideStack ? max(1u, (kWideStack - sp) / kNarrowPart) : 1u;
+    const uint32_t k = min(full ? min(32u, narrow) : 32u, sp);
+    popped += k;
     if (lane < k) {
       const uint2 pr = stack[sp - 1 - lane];
       a = pr.x;
@@ -377,11 +407,21 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
       push[3] = !la && !lb && overlap6(p1, q1);
     }
     // pushed in reverse of the recursion's order
+    uint32_t mask[4], total = 0;
 #pragma unroll
-    for (int c = 3; c >= 0; --c) {
-      const uint32_t mask = __ballot_sync(kAll, push[c]);
-      if (push[c]) stack[sp + __popc(mask & lt)] = make_uint2(xa[c & 1], xb[c >> 1]);
-      sp += __popc(mask);
+    for (int c = 0; c < 4; ++c) {
+      mask[c] = __ballot_sync(kAll, push[c]);
+      total += __popc(mask[c]);
+    }
+    if (sp + total > kPairStack) {  // beyond 64 levels of a search by single pairs
+      if (lane == 0) raise_status(status, kStatusStackOverflow);
+      sp = 0;
+    } else {
+#pragma unroll
+      for (int c = 3; c >= 0; --c) {
+        if (push[c]) stack[sp + __popc(mask[c] & lt)] = make_uint2(xa[c & 1], xb[c >> 1]);
+        sp += __popc(mask[c]);
+      }
     }
     __syncwarp();
     if (nleaf >= 32) {
@@ -391,6 +431,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
       __syncwarp();
     }
   }
+  if (lane == 0 && popped != 0) atomicAdd(rl.popped, static_cast<unsigned long long>(popped));
   if (lane < nleaf) {
     const uint2 pr = leaf[lane];
     report_pair(m, pr.x, pr.y, capacity, pairs, segments, count, status);
@@ -403,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
 namespace {
 
 constexpr uint32_t kRounds = 64;       // rounds between two clearings of the counters
-constexpr size_t kHeaderBytes = 1024;  // [start pairs given out, length of the list] per round
+constexpr size_t kHeaderBytes = 1024;  // [start pairs given out, length of the list] per round, pairs popped
 
 int round_grid() {
   static int cached[64] = {0};
@@ -430,7 +471,7 @@ int launch_self_intersection(cudaStream_t s, const MeshView& m, uint32_t capacit
                              uint32_t* count, void* scratch, size_t scratch_bytes, uint32_t* status) {
   if (m.num_tri < 2) return 0;
   uint32_t* counters = static_cast<uint32_t*>(scratch);  // 2 * kRounds words and the last list's length
-  static_assert((2 * kRounds + 2) * sizeof(uint32_t) <= kHeaderBytes, "counters");
+  static_assert((2 * kRounds + 2) * sizeof(uint32_t) <= kHeaderBytes - 8, "counters");
   const uint64_t cap = (scratch_bytes - kHeaderBytes) / (2 * sizeof(uint2));
   uint2* list[2] = {reinterpret_cast<uint2*>(static_cast<char*>(scratch) + kHeaderBytes), nullptr};
   list[1] = list[0] + cap;
@@ -447,7 +488,7 @@ int launch_self_intersection(cudaStream_t s, const MeshView& m, uint32_t capacit
     if (r == 0 && round > 0) {  // the list's length moves to the front, the rest is cleared
       if (cudaMemcpyAsync(counters + 1, counters + 2 * kRounds + 1, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s) !=
               cudaSuccess ||
-          cudaMemsetAsync(counters + 2, 0, kHeaderBytes - 8, s) != cudaSuccess ||
+          cudaMemsetAsync(counters + 2, 0, 2 * kRounds * sizeof(uint32_t), s) != cudaSuccess ||
           cudaMemsetAsync(counters, 0, 4, s) != cudaSuccess)
         return -1;
     }
@@ -458,6 +499,8 @@ int launch_self_intersection(cudaStream_t s, const MeshView& m, uint32_t capacit
     rl.next = list[round & 1];
     rl.num_next = counters + 2 * (r + 1) + 1;
     rl.next_cap = static_cast<uint32_t>(cap < 0x7fffffffu ? cap : 0x7fffffffu);
+    rl.popped = reinterpret_cast<unsigned long long*>(static_cast<char*>(scratch) + kHeaderBytes - 8);
+    rl.most = 2ull * m.num_tri * m.num_tri;
     // the first round of a small mesh has no more warps than start pairs
     const int grid = round == 0 && need < static_cast<uint32_t>(full) ? static_cast<int>(need) : full;
     if (reinterpret_cast<uintptr_t>(m.aabb) % 8 == 0)
