@@ -204,8 +204,8 @@ __device__ __forceinline__ void report_pair(const MeshView& m, uint32_t a0, uint
 // threads: 4.24 ms for two crossing tori of 260,084 triangles in all, against
 // 0.33 ms for the four rounds here.
 constexpr uint32_t kWarpsPerBlock = kThreads / 32;
-constexpr uint32_t kPairStack = 784;   // node pairs on a warp's stack (the most that leaves 8 blocks per SM)
-constexpr uint32_t kWideStack = 592;   // of them while pairs are popped several at a time
+constexpr uint32_t kPairStack = 704;   // node pairs on a warp's stack (784 cost two crossing tori 2%)
+constexpr uint32_t kWideStack = 512;   // of them while pairs are popped several at a time
 constexpr uint32_t kLeafBuffer = 64;   // leaf pairs waiting for their test
 // Every so many steps a warp looks whether the round's start pairs are all
 // given out; if so warps are running idle, and it hands its own pairs to the
@@ -214,7 +214,11 @@ constexpr uint32_t kLeafBuffer = 64;   // leaf pairs waiting for their test
 // side took 1.49, 1.18, 1.03 and 1.08 ms for 8, 16, 32 and 64 steps.
 constexpr uint32_t kRoundSteps = 32;
 
-constexpr uint32_t kAloneLooks = 2048;  // looks of a search that nothing ends
+// Looks without handing over after which a warp counts its pairs for all, and
+// after which it hands over although others are still busy: a search that does
+// not end shows in the one or in the number of rounds.  (Every warp adding its
+// count once a round cost two crossing tori 18 us of 380.)
+constexpr uint32_t kCountLooks = 64, kAloneLooks = 2048;
 
 // A warp whose next list is full goes on alone, and must not run out of stack:
 // popping 32 pairs whose boxes all overlap pushes up to 128.  From then on it pops
@@ -234,8 +238,8 @@ struct RoundList {
   uint2* next;         // the next round's list
   uint32_t* num_next;
   uint32_t next_cap;
-  // pairs popped over all rounds, and how many there can be: a tree has each pair
-  // of nodes once, so a search beyond that is one without an end (a cycle)
+  // pairs popped by searches that go on for long, and how many there can be: a
+  // tree has each pair of nodes once, so a search beyond that does not end (a cycle)
   unsigned long long* popped;
   unsigned long long most;
 };
@@ -344,18 +348,18 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
       // for which the rounds are the bound) is handed over all the same
       uint32_t taken = 0;
       bool endless = false;
-      if (lane == 0) {
-        taken = *reinterpret_cast<volatile uint32_t*>(rl.take);
-        endless = atomicAdd(rl.popped, static_cast<unsigned long long>(popped)) + popped > rl.most;
-      }
-      popped = 0;
-      if (__any_sync(kAll, endless)) {
-        bad = true;
-        break;
+      if (lane == 0) taken = *reinterpret_cast<volatile uint32_t*>(rl.take);
+      if (alone >= kCountLooks) {
+        if (lane == 0) endless = atomicAdd(rl.popped, static_cast<unsigned long long>(popped)) + popped > rl.most;
+        popped = 0;
+        if (__any_sync(kAll, endless)) {
+          bad = true;
+          break;
+        }
       }
       taken = __shfl_sync(kAll, taken, 0);
       if ((taken >= num_start || alone >= kAloneLooks) && hand_over(rl, stack, sp, sp, true, lane) != 0) {
-        alone = 0;
+        alone = popped = 0;
         full = full && sp + 96 > kWideStack;
         continue;
       }
@@ -406,22 +410,22 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
       push[2] = !lb && overlap6(p0, q1);
       push[3] = !la && !lb && overlap6(p1, q1);
     }
-    // pushed in reverse of the recursion's order
-    uint32_t mask[4], total = 0;
+    if (sp + 4 * k > kPairStack) {  // a search by single pairs; beyond 64 levels of it
+      uint32_t total = 0;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      mask[c] = __ballot_sync(kAll, push[c]);
-      total += __popc(mask[c]);
-    }
-    if (sp + total > kPairStack) {  // beyond 64 levels of a search by single pairs
-      if (lane == 0) raise_status(status, kStatusStackOverflow);
-      sp = 0;
-    } else {
-#pragma unroll
-      for (int c = 3; c >= 0; --c) {
-        if (push[c]) stack[sp + __popc(mask[c] & lt)] = make_uint2(xa[c & 1], xb[c >> 1]);
-        sp += __popc(mask[c]);
+      for (int c = 0; c < 4; ++c) total += __popc(__ballot_sync(kAll, push[c]));
+      if (sp + total > kPairStack) {
+        if (lane == 0) raise_status(status, kStatusStackOverflow);
+        sp = 0;
+        push[0] = push[1] = push[2] = push[3] = false;
       }
+    }
+    // pushed in reverse of the recursion's order
+#pragma unroll
+    for (int c = 3; c >= 0; --c) {
+      const uint32_t mask = __ballot_sync(kAll, push[c]);
+      if (push[c]) stack[sp + __popc(mask & lt)] = make_uint2(xa[c & 1], xb[c >> 1]);
+      sp += __popc(mask);
     }
     __syncwarp();
     if (nleaf >= 32) {
@@ -431,7 +435,6 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
       __syncwarp();
     }
   }
-  if (lane == 0 && popped != 0) atomicAdd(rl.popped, static_cast<unsigned long long>(popped));
   if (lane < nleaf) {
     const uint2 pr = leaf[lane];
     report_pair(m, pr.x, pr.y, capacity, pairs, segments, count, status);

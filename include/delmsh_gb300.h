@@ -361,7 +361,7 @@ int dm_pix2tri_interpolate_bwd_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t 
  * pierces the other triangle.  *count (device u32) receives the number of
  * pairs, which may exceed `capacity`, in which case only `capacity` pairs are
  * written (call again with a larger buffer).  The list is unordered.  The
- * search keeps one 784-entry stack of node pairs per warp (status bit 2 if one
+ * search keeps one 704-entry stack of node pairs per warp (status bit 2 if one
  * overflows) and runs in rounds that rebalance the remaining work; every fourth
  * reads the next round's size back to the host, so the call synchronizes the
  * stream.  Its working memory (16 MB per million triangles, at least 16 MB)
