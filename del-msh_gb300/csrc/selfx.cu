@@ -446,6 +446,9 @@ __global__ void __launch_bounds__(kThreads, 8) k_selfx_round(MeshView m, RoundLi
 
 namespace {
 
+// The rounds have run out with pairs left.
+__global__ void k_selfx_unfinished(uint32_t* status) { raise_status(status, kStatusStackOverflow); }
+
 constexpr uint32_t kRounds = 64;       // rounds between two clearings of the counters
 constexpr size_t kHeaderBytes = 1024;  // [start pairs given out, length of the list] per round, pairs popped
 
@@ -482,11 +485,14 @@ int launch_self_intersection(cudaStream_t s, const MeshView& m, uint32_t capacit
   const uint32_t need = (m.num_tri - 1 + kThreads - 1) / kThreads;
   if (cudaMemsetAsync(counters, 0, kHeaderBytes, s) != cudaSuccess) return -1;
   // Rounds until no warp hands work on.  Each round either finishes its warps'
-  // work or splits it, so there are few (bounded here).  The length of a
-  // round's list stays on the device: kAhead rounds are launched between two
-  // looks at it, an empty one costs 2 us and a look 15.
+  // work or splits it, so there are few, but a search down a chain of n links by
+  // itself (n equal codes) takes n / kRoundSteps of them; the bound is for trees
+  // with cycles.  The length of a round's list stays on the device: kAhead rounds
+  // are launched between two looks at it, an empty one costs 2 us and a look 15.
   constexpr uint32_t kAhead = 4;
-  for (uint32_t round = 0; round < 4000; ++round) {
+  const uint32_t max_round = 4000 + m.num_tri / 16 / kAhead * kAhead;
+  static_assert(4000 % kAhead == 0, "the last round is looked at");
+  for (uint32_t round = 0; round < max_round; ++round) {
     const uint32_t r = round % kRounds;
     if (r == 0 && round > 0) {  // the list's length moves to the front, the rest is cleared
       if (cudaMemcpyAsync(counters + 1, counters + 2 * kRounds + 1, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s) !=
@@ -517,6 +523,7 @@ int launch_self_intersection(cudaStream_t s, const MeshView& m, uint32_t capacit
       if (n == 0) return 0;
     }
   }
+  k_selfx_unfinished<<<1, 1, 0, s>>>(status);
   return 0;
 }
 

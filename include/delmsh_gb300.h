@@ -362,7 +362,8 @@ int dm_pix2tri_interpolate_bwd_ex(uint64_t stream_ptr, uint32_t img_w, uint32_t 
  * pairs, which may exceed `capacity`, in which case only `capacity` pairs are
  * written (call again with a larger buffer).  The list is unordered.  The
  * search keeps one 704-entry stack of node pairs per warp (status bit 2 if one
- * overflows) and runs in rounds that rebalance the remaining work; every fourth
+ * overflows or the search of a malformed tree does not end, bit 4 if it visits
+ * more pairs than a tree has) and runs in rounds that rebalance the remaining work; every fourth
  * reads the next round's size back to the host, so the call synchronizes the
  * stream.  Its working memory (16 MB per million triangles, at least 16 MB)
  * comes from cudaMallocAsync, or from the caller in the _ex form.
