@@ -114,7 +114,8 @@ void launch_cast_pixels(cudaStream_t s, uint32_t img_w, uint32_t img_h, const Ca
   job.row_major = camera.row_major;
   if (camera.host) memcpy(job.t_value, camera.host, sizeof(job.t_value));
   job.o = o;
-  cast_job(s, job, sc, m.num_tri, status, busy);
+  if (busy) cast_job<SingleJob, true>(s, job, sc, m.num_tri, status);
+  else cast_job(s, job, sc, m.num_tri, status);
 }
 
 void launch_cast_rays(cudaStream_t s, uint32_t num_ray, const float* ray_org, const float* ray_dir,
@@ -125,7 +126,8 @@ void launch_cast_rays(cudaStream_t s, uint32_t num_ray, const float* ray_org, co
   job.ray_org = ray_org;
   job.ray_dir = ray_dir;
   job.o = o;
-  cast_job(s, job, sc, m.num_tri, status, busy);
+  if (busy) cast_job<SingleJob, true>(s, job, sc, m.num_tri, status);
+  else cast_job(s, job, sc, m.num_tri, status);
 }
 
 }  // namespace dm

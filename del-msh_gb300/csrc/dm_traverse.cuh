@@ -429,10 +429,13 @@ struct Parked {
 // registers keep 36 warps resident where 64 keep 32.  For the batch that pays,
 // 64 / 56 / 48 registers: 1220 / 1173 / 1195 us; one mesh's cast spills more and
 // is also held by single rays: 2M triangles at 1920 x 1080 431 / 440 / 446 us,
-// 16,384 rays 136 / 143 / 144 us.  The loop after the work has run
-// out is a second copy of the phases: with one loop for both, the parking code
-// cost the first one 100 bytes of spills (batched cast 1.26 -> 1.48 ms).
-template <typename Job, int kThreads, int kStack>
+// 16,384 rays 136 / 143 / 144 us.
+// With kPark the loop after the work has run out is a second copy of the phases:
+// with one loop for both, the parking code cost the first one 100 bytes of spills
+// (batched cast 1.26 -> 1.48 ms).  Without it, for a GPU that is busy with other
+// requests' kernels (see launch_tiers), one loop does both: with two, a server's
+// capacity was 6,220 requests/s, with one it is 7,270 (512 meshes, 8 in flight).
+template <typename Job, int kThreads, int kStack, bool kPark>
 __global__ void __launch_bounds__(kThreads, 65536 / (Job::kCastRegs * kThreads)) k_cast_persistent(Job job, uint32_t* work_counter,
                                                                                  uint32_t* ovf_list,
                                                                                  uint32_t* ovf_count,
@@ -472,8 +475,12 @@ __global__ void __launch_bounds__(kThreads, 65536 / (Job::kCastRegs * kThreads))
         }
       }
     }
-    if (exhausted) break;
-    if (__all_sync(kAll, state == kLaneIdle)) continue;
+    if (kPark && exhausted) break;
+    if (__all_sync(kAll, state == kLaneIdle)) {
+      if (exhausted) break;
+      continue;
+    }
+    const uint32_t leaf_min = exhausted ? 1u : mins.leaf, ascend_min = exhausted ? 1u : mins.ascend;
     // Up to kInnerSteps node entries per iteration: the warp's votes and
     // phase decisions are paid once for several entries, and a lane that
     // leaves the inner phase early waits for the others' entries.
@@ -482,14 +489,17 @@ __global__ void __launch_bounds__(kThreads, 65536 / (Job::kCastRegs * kThreads))
       if (state == kLaneInner) state = phase_inner(m, r, stack, kStack, s, bad);
     uint32_t inner = __ballot_sync(kAll, state == kLaneInner);
     const uint32_t leaf = __ballot_sync(kAll, state == kLaneLeaf);
-    if (leaf != 0u && (inner == 0u || static_cast<uint32_t>(__popc(leaf)) >= mins.leaf)) {
+    if (leaf != 0u && (inner == 0u || static_cast<uint32_t>(__popc(leaf)) >= leaf_min)) {
       if (state == kLaneLeaf) state = phase_leaf(m, r, s, bad);
       inner = __ballot_sync(kAll, state == kLaneInner);
     }
     const uint32_t asc = __ballot_sync(kAll, state == kLaneAscend);
-    if (asc != 0u && (inner == 0u || static_cast<uint32_t>(__popc(asc)) >= mins.ascend)) {
+    if (asc != 0u && (inner == 0u || static_cast<uint32_t>(__popc(asc)) >= ascend_min)) {
       if (state == kLaneAscend) state = phase_ascend(m, r, stack, s, bad);
     }
+    if (!kPark && exhausted && state == kLaneInner && s.steps > mins.long_steps &&
+        long_chain_at(m, s.node, s.left, s.right))
+      state = kLaneOverflow;
     if (state == kLaneDone) {
       job.write(out, m, r, s.best);
       state = kLaneIdle;
@@ -497,6 +507,10 @@ __global__ void __launch_bounds__(kThreads, 65536 / (Job::kCastRegs * kThreads))
       ovf_list[atomicAdd(ovf_count, 1u)] = work;
       state = kLaneIdle;
     }
+  }
+  if constexpr (!kPark) {
+    if (bad) raise_status(status, kStatusBadIndex);
+    return;
   }
   // The warp has no more rays to take: a waiting lane would only lengthen its
   // longest ray, so every phase runs whenever a lane needs it.  A ray past the
@@ -1195,7 +1209,7 @@ __global__ void __launch_bounds__(kTeamThreads, kTailBlocks) k_cast_tail(Job job
 
 // Number of resident blocks of a persistent kernel instantiation on the
 // current device.
-template <typename Job, int kThreads, int kStack>
+template <typename Job, int kThreads, int kStack, bool kPark>
 inline int persistent_grid() {
   static int cached[64] = {0};
   int dev = 0;
@@ -1204,7 +1218,8 @@ inline int persistent_grid() {
   if (cached[dev] == 0) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cast_persistent<Job, kThreads, kStack>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cast_persistent<Job, kThreads, kStack, kPark>, kThreads,
+                                                  0);
     cached[dev] = (sms > 0 ? sms : 152) * (per_sm > 0 ? per_sm : 1);
   }
   return cached[dev];
@@ -1232,11 +1247,6 @@ inline uint32_t park_steps(uint32_t num_work) {
   return kParkSteps + kParkMore * doublings;
 }
 
-// `busy`: the GPU has other work to do beside this cast (a server with requests
-// in flight).  Then the cast's own latency counts for less than the issue slots
-// it takes: warps are filled and nothing is parked, as helpers also search
-// subtrees that turn out not to be needed.  64 requests in flight at once took
-// 4.65 ms so and 5.01 ms with parking.
 // Zeroes a cast's counters.  A kernel instead of a copy-engine memset, so that
 // the persistent cast's blocks are resident when it ends.
 static __global__ void k_cast_begin(uint32_t* counters) {
@@ -1245,17 +1255,21 @@ static __global__ void k_cast_begin(uint32_t* counters) {
   if (threadIdx.x < kCastCounterBytes / sizeof(uint32_t)) counters[threadIdx.x] = 0u;
 }
 
-template <typename Job, int kThreads, int kStack>
-inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, bool busy,
-                         uint32_t* status) {
-  int grid = persistent_grid<Job, kThreads, kStack>();
+// `busy`: the GPU has other work to do beside this cast (a server with requests
+// in flight).  Then the cast's own latency counts for less than the issue slots
+// it takes: warps are filled and nothing is parked, as helpers also search
+// subtrees that turn out not to be needed.  64 requests in flight at once took
+// 4.65 ms so and 5.01 ms with parking.
+template <typename Job, int kThreads, int kStack, bool kBusy>
+inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, uint32_t* status) {
+  int grid = persistent_grid<Job, kThreads, kStack, !kBusy>();
   const uint32_t warps = static_cast<uint32_t>(grid) * (kThreads / 32);
   // few rays are spread over all warps, so that a warp has fewer phases to run
   // one after the other and more lanes to help in the split tier: 16,384 rays by
   // 32, 8, 4, 2 per warp: 135, 126, 131, 134 us.  From about 8 per warp on there
   // is no gain (65,536 rays by 14: 177 against 171 us for build and cast).
   const uint32_t share =
-      job.num_work <= 8 * warps && !busy ? (job.num_work + warps - 1) / warps : 32u;
+      job.num_work <= 8 * warps && !kBusy ? (job.num_work + warps - 1) / warps : 32u;
   const uint32_t needed = ((job.num_work + share - 1) / share + kThreads / 32 - 1) / (kThreads / 32);
   if (static_cast<uint32_t>(grid) > needed) grid = static_cast<int>(needed);
   const Tuning t = get_tuning();
@@ -1267,7 +1281,7 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   // 1231, 1253 us).
   const uint32_t refill = min(t.cast_refill_min * Job::kRefillHalves / 2u, 32u);
   const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps,
-                       busy ? kUMax : park_steps(job.num_work), share};
+                       kBusy ? kUMax : park_steps(job.num_work), share};
   TailArgs a;
   a.parked.rays = static_cast<uint4*>(sc.pool);
   a.parked.count = sc.counters + 5;
@@ -1288,7 +1302,7 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   a.long_steps = t.cast_long_steps;
   a.status = status;
   launch_pdl(k_cast_begin, dim3(1), dim3(32), 0, s, sc.counters);
-  launch_pdl(k_cast_persistent<Job, kThreads, kStack>, dim3(grid), dim3(kThreads), 0, s, job, sc.counters, sc.list1,
+  launch_pdl(k_cast_persistent<Job, kThreads, kStack, !kBusy>, dim3(grid), dim3(kThreads), 0, s, job, sc.counters, sc.list1,
              sc.counters + 1, status, mins, a.parked);
   launch_pdl(k_cast_tail<Job, kStack>, dim3(152 * kTailBlocks), dim3(kTeamThreads), 0, s, job, a);
 }
@@ -1300,16 +1314,15 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
 // [4] rays taken by the team tier, [5] rays parked, [6] parked rays taken, [7]
 // blocks done.  The first tier's block size and on-chip stack depth come from
 // the current Tuning (kCastVariants lists the choices).
-template <typename Job>
-inline void cast_job(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, uint32_t* status,
-                     bool busy = false) {
+template <typename Job, bool kBusy = false>
+inline void cast_job(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, uint32_t* status) {
   if (job.num_work == 0) return;
   const Tuning t = get_tuning();
-  if (t.cast_threads == 64 && t.cast_stack == 64) launch_tiers<Job, 64, 64>(s, job, sc, max_tri, busy, status);
-  else if (t.cast_threads == 256 && t.cast_stack == 64) launch_tiers<Job, 256, 64>(s, job, sc, max_tri, busy, status);
-  else if (t.cast_threads == 128 && t.cast_stack == 32) launch_tiers<Job, 128, 32>(s, job, sc, max_tri, busy, status);
-  else if (t.cast_threads == 128 && t.cast_stack == 96) launch_tiers<Job, 128, 96>(s, job, sc, max_tri, busy, status);
-  else launch_tiers<Job, 128, 64>(s, job, sc, max_tri, busy, status);
+  if (t.cast_threads == 64 && t.cast_stack == 64) launch_tiers<Job, 64, 64, kBusy>(s, job, sc, max_tri, status);
+  else if (t.cast_threads == 256 && t.cast_stack == 64) launch_tiers<Job, 256, 64, kBusy>(s, job, sc, max_tri, status);
+  else if (t.cast_threads == 128 && t.cast_stack == 32) launch_tiers<Job, 128, 32, kBusy>(s, job, sc, max_tri, status);
+  else if (t.cast_threads == 128 && t.cast_stack == 96) launch_tiers<Job, 128, 96, kBusy>(s, job, sc, max_tri, status);
+  else launch_tiers<Job, 128, 64, kBusy>(s, job, sc, max_tri, status);
 }
 
 }  // namespace dm
