@@ -710,6 +710,7 @@ __device__ __forceinline__ void test_links(const MeshView& m, const Ray& r, uint
     const uint32_t cut = __ballot_sync(kWarpAll, i < n && !(flags[q] & 2u));  // links that do not look at x
     uint32_t todo = __ballot_sync(kWarpAll, i < n && (flags[q] & 2u) && h.id != kUMax) | cut;
     if (cut != 0u) {  // what comes before the last of them is lost
+      __syncwarp();  // their entries are written over (a ballot orders no memory)
       todo &= 0xffffffffu << (31 - __clz(cut));
       num = 0;
       has_cut = 1;
