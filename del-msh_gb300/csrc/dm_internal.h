@@ -306,7 +306,7 @@ struct CastOut {
   float* hit_bc;      // optional, 3 per ray (1-u-v, u, v)
 };
 
-constexpr size_t kCastCounterBytes = 32;
+constexpr size_t kCastCounterBytes = 256;
 
 struct CastScratch {
   uint32_t* counters;  // kCastCounterBytes (see cast_job)

@@ -410,6 +410,18 @@ struct Parked {
   uint4* rays;  // per ray: {work, node, left, right}, {sp, steps, best}, the frames
   uint32_t* count;
   uint32_t capacity, stride;
+  __device__ __forceinline__ uint32_t work(uint32_t i) const { return rays[static_cast<size_t>(i) * stride].x; }
+  // The first of a block's list of rays that the split tier hands over (linked by
+  // their second word), or kUMax; by many threads of the block at a time.
+  __device__ __forceinline__ uint32_t take_handed(uint32_t* head) const {
+    uint32_t i = *reinterpret_cast<volatile uint32_t*>(head);
+    while (i != kUMax) {
+      const uint32_t seen = atomicCAS(head, i, rays[static_cast<size_t>(i) * stride + 1].x);
+      if (seen == i) break;
+      i = seen;
+    }
+    return i;
+  }
 };
 
 // Persistent warps with per-lane ray refill, run in phases.  Each lane holds
@@ -606,23 +618,27 @@ struct FoldShared {
   uint32_t first[2];  // chain_last: the first record of the warp's that is no link
 };
 
-// The warps that cast one ray together: the whole block, or a warp alone.  The
-// two sides of FoldShared are used in turn over all chains of the kernel, so
-// that a warp writes a side again only after a meeting of the team that the
-// others reach when they have read it.
+// The warps that cast one ray together: the whole block, or a warp alone (known when
+// compiled: one function for both took 5% longer for a soup's build and cast).  The
+// two sides of FoldShared are used in turn over all chains of a ray, so that a warp
+// writes a side again only after a meeting of the team that the others reach when
+// they have read it.
+template <bool kSolo>
 struct Team {
+  static constexpr uint32_t warps = kSolo ? 1u : kTeamWarps;
   FoldShared* sh;  // the team's first warp's
-  uint32_t rank, warps, lane;
+  uint32_t rank, lane;
   mutable uint32_t scan_side, fold_side;
   __device__ __forceinline__ void sync() const {
-    if (warps > 1) __syncthreads();
-    else __syncwarp();
+    if constexpr (kSolo) __syncwarp();
+    else __syncthreads();
   }
 };
 
 // The last link of the chain starting at link c0 (the same in every lane of the
 // team), 256 records per warp and round (8 per lane).
-__device__ __forceinline__ uint32_t chain_last(const MeshView& m, uint32_t c0, const Team& tm) {
+template <bool kSolo>
+__device__ __forceinline__ uint32_t chain_last(const MeshView& m, uint32_t c0, const Team<kSolo>& tm) {
   const uint32_t num_branch = m.num_tri - 1;
   uint32_t last = c0;
   for (;;) {
@@ -650,7 +666,7 @@ __device__ __forceinline__ uint32_t chain_last(const MeshView& m, uint32_t c0, c
       const uint32_t l0 = static_cast<uint32_t>(__ffs(fail)) - 1u;
       mine = 8 * l0 + __shfl_sync(kWarpAll, first_bad, l0);
     }
-    if (tm.warps == 1) {
+    if constexpr (kSolo) {
       if (mine < 256) return last + mine;
     } else {
       if (tm.lane == 0) tm.sh[tm.rank].first[side] = mine;
@@ -726,7 +742,8 @@ __device__ __forceinline__ void test_links(const MeshView& m, const Ray& r, uint
 }
 
 // The links of a round applied to x, the warps' parts from the far end on.
-__device__ __forceinline__ Hit apply_links(const Team& tm, uint32_t side, Hit x) {
+template <bool kSolo>
+__device__ __forceinline__ Hit apply_links(const Team<kSolo>& tm, uint32_t side, Hit x) {
   uint32_t w0 = 0;
   for (uint32_t w = 1; w < tm.warps; ++w)
     if (tm.sh[w].cut[side]) w0 = w;
@@ -746,9 +763,9 @@ __device__ __forceinline__ Hit apply_links(const Team& tm, uint32_t side, Hit x)
 // phase_inner, except that a branch starting a chain of at least kFoldMin
 // links pushes a fold frame {c0 | bit, c1 | bit, saved} and searches the
 // chain's tail (if its box is hit) with a fresh result.
-template <typename StackT>
+template <typename StackT, bool kSolo>
 __device__ __forceinline__ int phase_inner_team(const MeshView& m, const Ray& r, StackT stack, uint32_t cap, Trav& s,
-                                                bool& bad, const Team& tm) {
+                                                bool& bad, const Team<kSolo>& tm) {
   if (s.right != kUMax && is_link(m, s.node, s.left, s.right)) {
     const uint32_t c0 = s.node, c1 = chain_last(m, c0, tm);
     if (c1 - c0 + 1 >= kFoldMin) {
@@ -776,10 +793,11 @@ constexpr uint32_t kChainPrefetch = 8;  // groups of 32 links per warp prefetche
 
 // Fold frames {c0 | bit, c1 | bit, saved}: the tail's result (the current
 // one) is folded through the chain, and the chain's result into `saved`.
+template <bool kSolo>
 struct ChainFold {
   const MeshView& m;
   const Ray& r;
-  const Team& tm;
+  const Team<kSolo>& tm;
   bool* bad;
   __device__ __forceinline__ int operator()(const uint4& f, Trav& s) const {
     if (!((f.x & kChainBit) && (f.y & kChainBit))) return 0;
@@ -820,12 +838,12 @@ struct ChainFold {
   }
 };
 
-template <typename StackT>
+template <typename StackT, bool kSolo>
 __device__ __forceinline__ int trav_step_team(const MeshView& m, const Ray& r, StackT stack, uint32_t cap, Trav& s,
-                                              bool& bad, const Team& tm) {
+                                              bool& bad, const Team<kSolo>& tm) {
   int st = phase_inner_team(m, r, stack, cap, s, bad, tm);
   if (st == kLaneLeaf) st = phase_leaf(m, r, s, bad);
-  if (st == kLaneAscend) st = phase_ascend(m, r, stack, s, bad, ChainFold{m, r, tm, &bad});
+  if (st == kLaneAscend) st = phase_ascend(m, r, stack, s, bad, ChainFold<kSolo>{m, r, tm, &bad});
   return st == kLaneInner ? kStepContinue : (st == kLaneOverflow ? kStepOverflow : kStepDone);
 }
 
@@ -851,8 +869,8 @@ __device__ __forceinline__ int trav_step_team(const MeshView& m, const Ray& r, S
 // rays keep their time (4.2M rays on 1,024 small meshes, at most 100 entries:
 // 1.26 -> 1.23 ms).
 // A ray that runs into a long chain or out of stack is linked into the block's
-// own list (`handed`, by parked index; the next one in its second word) and cast
-// by the block as a team afterwards.
+// own list (`handed`: the first by parked index, and how many; the next one in its
+// second word) and cast by the block's team or teams afterwards.
 template <typename Job, int kStack>
 __device__ __forceinline__ void cast_split(const Job& job, const float* smem, const Parked& parked, uint32_t num,
                                            uint32_t* take, uint2* sh_deal, uint32_t* handed, uint32_t long_steps,
@@ -1006,8 +1024,10 @@ __device__ __forceinline__ void cast_split(const Job& job, const float* smem, co
         if (more == over) break;
         over = more;
       }
-      if ((over >> lane & 1u) && parent == kUMax)
+      if ((over >> lane & 1u) && parent == kUMax) {
         parked.rays[static_cast<size_t>(slot) * parked.stride + 1].x = atomicExch(handed, slot);
+        atomicAdd(handed + 1, 1u);
+      }
       drop |= over;
     }
     if (drop != 0u) {  // and with a lane all that help it
@@ -1027,36 +1047,57 @@ __device__ __forceinline__ void cast_split(const Job& job, const float* smem, co
   if (bad) raise_status(status, kStatusBadIndex);
 }
 
-// Re-casts the work indices list_in[0 .. num) by one block, a thread per ray,
-// with stacks carved from the pool.  cap_fixed == 0 chooses the capacity from
-// the number of rays to process.
-template <typename Job>
-__device__ __noinline__ void cast_deep(const Job& job, const float* smem, const uint32_t* list_in, uint32_t num,
-                                       uint32_t* list_out, uint32_t* count_out, uint4* pool, uint64_t pool_frames,
-                                       uint32_t cap_fixed, uint32_t max_tri, uint32_t* status) {
-  uint64_t cap = cap_fixed;
-  if (cap == 0) {
-    cap = pool_frames / num;
-    if (cap < 256) cap = 256;
-    const uint64_t cap_max = 2ull * max_tri;  // never more than the deepest possible tree needs
-    if (cap > cap_max) cap = cap_max;
+// Rays of the team tier's list linked into lists of those to be cast again: such a
+// list is the index of its first ray, or kUMax.
+struct RayLinks {
+  uint32_t* team_list;  // work indices
+  uint32_t* next;       // per entry of team_list
+  __device__ __forceinline__ uint32_t work(uint32_t id) const {
+    return *reinterpret_cast<const volatile uint32_t*>(team_list + id);
   }
+  // By many at a time; read only after all of them.
+  __device__ __forceinline__ void push(uint32_t* head, uint32_t id) const { next[id] = atomicExch(head, id); }
+  // For a ray that was parked, and so is in no list yet: `id` is a free entry.
+  __device__ __forceinline__ uint32_t append(uint32_t id, uint32_t w) const {
+    team_list[id] = w;
+    return id;
+  }
+  // By the threads of one block at a time; no ray is pushed meanwhile.
+  __device__ __forceinline__ uint32_t pop(uint32_t* head) const {
+    uint32_t id = *reinterpret_cast<volatile uint32_t*>(head);
+    while (id != kUMax) {
+      const uint32_t seen = atomicCAS(head, id, *reinterpret_cast<volatile uint32_t*>(next + id));
+      if (seen == id) break;
+      id = seen;
+    }
+    return id;
+  }
+};
+
+// Re-casts a list of rays by one block, a thread per ray, with stacks of `cap`
+// frames (of pool_frames, if that is less) carved from pool[0 .. pool_frames) and
+// more[0 .. more_frames).
+template <typename Job>
+__device__ __noinline__ void cast_deep(const Job& job, const float* smem, const RayLinks& links, uint32_t* list,
+                                       uint4* pool, uint64_t pool_frames, uint4* more, uint64_t more_frames,
+                                       uint64_t cap, uint32_t* status) {
   if (cap > pool_frames) cap = pool_frames;
-  uint64_t slots = pool_frames / cap;
-  if (slots > blockDim.x) slots = blockDim.x;
-  const uint32_t slot = threadIdx.x;
-  if (slot >= slots) return;
+  const uint64_t slot = threadIdx.x, here = pool_frames / cap;
+  const bool has_stack = slot < here + more_frames / cap;
   uint4 ring[kDeepRing];
   uint32_t lo = 0;
-  const RingStack<kDeepRing> st{ring, pool + slot * cap, &lo};
+  const RingStack<kDeepRing> st{ring, slot < here ? pool + slot * cap : more + (slot - here) * cap, &lo};
   bool bad = false;
-  for (uint64_t k = slot; k < num; k += slots) {
-    lo = 0;
-    const uint32_t w = list_in[k];
+  for (;;) {
+    // a warp's lanes start together: on their own they would stay apart, each of
+    // them with the loads of a step to itself
+    const uint32_t id = has_stack ? links.pop(list) : kUMax;
+    if (!__any_sync(kWarpAll, id != kUMax)) break;
     MeshView m{};
     Ray r{};
     uint32_t out = 0;
-    if (!job.fetch(w, smem, m, r, out)) continue;
+    if (id == kUMax || !job.fetch(links.work(id), smem, m, r, out)) continue;
+    lo = 0;
     Trav s{};
     int rc = kStepDone;
     if (trav_begin(m, r, s)) {
@@ -1066,8 +1107,6 @@ __device__ __noinline__ void cast_deep(const Job& job, const float* smem, const 
     }
     if (rc == kStepDone) {
       job.write(out, m, r, s.best);
-    } else if (list_out) {
-      list_out[atomicAdd(count_out, 1u)] = w;
     } else {
       raise_status(status, kStatusStackOverflow);
       job.write(out, m, r, Hit{INFINITY, kUMax});
@@ -1076,12 +1115,13 @@ __device__ __noinline__ void cast_deep(const Job& job, const float* smem, const 
   if (bad) raise_status(status, kStatusBadIndex);
 }
 
-// One ray cast by a team.  Every lane keeps the same stack (the ring in its own
-// local memory, the spilled frames at the same addresses of its warp's slice of
-// the pool); a ray whose frames outgrow the slice goes to list_out.
-template <typename Job>
-__device__ __noinline__ void cast_team(const Job& job, const float* smem, uint32_t w, const Team& tm, uint4* slice,
-                                       uint32_t cap, uint32_t* list_out, uint32_t* count_out, bool& bad) {
+// Ray `id` of the list cast by a team.  Every lane keeps the same stack (the ring in
+// its own local memory, the spilled frames at the same addresses of its warp's slice
+// of the pool); a ray whose frames outgrow the slice is linked into `over`.  All of the
+// team meet between two rays.
+template <bool kSolo, typename Job>
+__device__ __noinline__ void cast_team(const Job& job, const float* smem, uint32_t w, const Team<kSolo>& tm, uint4* slice,
+                                       uint32_t cap, uint32_t id, uint32_t* next, uint32_t* over, bool& bad) {
   uint4 ring[kDeepRing];
   uint32_t lo = 0;
   const RingStack<kDeepRing> st{ring, slice, &lo};
@@ -1098,7 +1138,7 @@ __device__ __noinline__ void cast_team(const Job& job, const float* smem, uint32
   }
   if (tm.rank == 0 && tm.lane == 0) {
     if (rc == kStepDone) job.write(out, m, r, s.best);
-    else list_out[atomicAdd(count_out, 1u)] = w;
+    else next[id] = atomicExch(over, id);
   }
 }
 
@@ -1106,28 +1146,31 @@ __device__ __noinline__ void cast_team(const Job& job, const float* smem, uint32
 struct TailArgs {
   Parked parked;          // rays for the split tier, in the first half of the pool
   uint32_t* parked_take;  // of them given out
-  const uint32_t* team_list;
+  RayLinks links;
   const uint32_t* team_count;
   uint32_t* team_take;
-  uint32_t* deep_list;   // rays whose frames outgrew a team's slice
-  uint32_t* deep_count;  // [0] of them, [1] of those that outgrew the next stack
-  uint32_t* last_list;
-  uint32_t* done;        // blocks that have finished
+  uint32_t* team_more;   // parked rays appended to team_list
+  uint32_t* deep;        // of all blocks, then per group: the rays whose frames outgrew a team's slice
+  uint32_t* done;        // of all blocks, then per group: those that have finished
   uint4* pool;
-  uint64_t pool_frames;
+  uint64_t pool_frames, slice_frames, group_frames;  // of all, of a team's warp, of a group
   uint32_t max_tri, long_steps;
   uint32_t* status;
 };
 
 // All tiers after the persistent cast in one launch: the split tier, then the
-// team tier, and the last block to finish casts what is left.  With a kernel for
-// each, an image without such rays paid three more launches: 6 us each of a
-// server's dispatcher thread.
+// team tier, then what outgrew a team's slice (some 570 frames and 64 more): trees
+// that are not of Morton codes, whose chains are folded.  The last block to finish
+// of each group of blocks casts the group's such rays, with stacks that are sure to
+// do, carved from the group's share of the pool; for trees so large that all groups
+// hold fewer stacks than one block has threads, the last block of all casts them,
+// with the whole pool.  With a kernel for each tier, an image without such rays paid
+// three more launches: 6 us each of a server's dispatcher thread.
 //
 // A team is a whole block while the rays are few, kTeamRays per block or
 // fewer: then the longest ray sets the kernel's end.  With more, their number
 // does, and each warp takes rays of its own.
-// Blocks a multiprocessor of the tail kernel: 6 (80 registers, 76 bytes of spills)
+// Blocks a multiprocessor of the tail kernel: 6 (80 registers, 80 bytes of spills)
 // let the split tier of large images hold more rays at once than 4 (124
 // registers) and cost the others nothing; 2M triangles at 1920 x 1080 with 4, 5,
 // 6, 8: 431, 432, 407, 416 us, 16,384 rays 135, 130, 132, 138 us, 512 x 512 of
@@ -1135,77 +1178,88 @@ struct TailArgs {
 // 709 us.
 constexpr uint32_t kTailBlocks = 6;
 constexpr uint32_t kTeamRays = 8;
+// Groups of blocks with a list of deep rays each.  Combs whose every level is a
+// frame, 4,096 rays, by the last block of all / by groups: 1,200 levels 77 / 5.0 ms,
+// 3,000 levels 143 / 16 ms.  (65,536 rays: 802 / 56 and 1,846 / 196 ms.)
+constexpr uint32_t kDeepGroups = 24;
+static_assert((7 + 2 * (1 + kDeepGroups)) * sizeof(uint32_t) <= kCastCounterBytes, "counters");
 template <typename Job, int kStack>
 __global__ void __launch_bounds__(kTeamThreads, kTailBlocks) k_cast_tail(Job job, TailArgs a) {
   __shared__ float smem[64];
   __shared__ FoldShared sh[kTeamWarps];
   __shared__ uint2 sh_deal[kTeamThreads];
-  __shared__ uint32_t sh_take, sh_handed;
+  __shared__ uint32_t sh_take, sh_handed[2];
   job.prepare(smem);
-  if (threadIdx.x == 0) sh_handed = kUMax;
+  if (threadIdx.x == 0) {
+    sh_handed[0] = kUMax;
+    sh_handed[1] = 0u;
+  }
   pdl_wait();
   __syncthreads();
   const uint32_t parked = min(*a.parked.count, a.parked.capacity), num = *a.team_count;
   if (parked == 0 && num == 0) return;
   if (parked != 0) {
-    cast_split<Job, kStack>(job, smem, a.parked, parked, a.parked_take, sh_deal, &sh_handed, a.long_steps, a.status);
+    cast_split<Job, kStack>(job, smem, a.parked, parked, a.parked_take, sh_deal, sh_handed, a.long_steps, a.status);
     __syncthreads();
   }
-  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31u;
-  // the teams' stacks lie in the pool's second half: parked rays may still be
-  // waiting in the first
-  const uint64_t half = a.pool_frames / 2, warps = static_cast<uint64_t>(gridDim.x) * kTeamWarps;
-  const uint64_t cap64 = min(static_cast<unsigned long long>(half / warps), 2ull * a.max_tri);
-  const uint32_t cap = static_cast<uint32_t>(cap64);
-  uint4* slice = a.pool + half + (static_cast<uint64_t>(blockIdx.x) * kTeamWarps + warp) * cap64;
-  bool bad = false;
-  const Team block{sh, warp, kTeamWarps, lane, 0u, 0u};
-  for (uint32_t i = sh_handed; i != kUMax;) {
-    const uint4* ray = a.parked.rays + static_cast<size_t>(i) * a.parked.stride;
-    const uint32_t w = ray[0].x;
-    i = ray[1].x;
-    cast_team(job, smem, w, block, slice, cap, a.deep_list, a.deep_count, bad);
-  }
-  __syncthreads();
-  if (num <= kTeamRays * gridDim.x) {
+  const uint32_t group = blockIdx.x % kDeepGroups;
+  const uint64_t half = a.pool_frames / 2, room = a.group_frames;  // a group's slices lie together
+  const uint32_t need = max(a.max_tri, 2u);  // no tree needs more frames than it has leaves
+  const bool grouped = room >= 6ull * need;  // 24 times 6: more than the threads of a block
+  uint32_t* const deep = a.deep + (grouped ? 1 + group : 0);
+  const RayLinks links = a.links;
+  // the split tier's rays of this block, then those of the list
+  for (uint32_t from_list = 0; from_list < 2; ++from_list) {
+    if (from_list ? num == 0 : sh_handed[1] == 0) continue;
+    const bool solo = from_list ? num > kTeamRays * gridDim.x : sh_handed[1] >= kTeamWarps;
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31u;
+    // the teams' stacks lie in the pool's second half: parked rays may still be
+    // waiting in the first
+    uint4* const slice =
+        a.pool + half + group * room + (blockIdx.x / kDeepGroups * kTeamWarps + warp) * a.slice_frames;
+    const uint32_t cap = static_cast<uint32_t>(min(a.slice_frames, static_cast<uint64_t>(need)));
+    const Team<true> one{sh + warp, 0u, lane, 0u, 0u};
+    const Team<false> all{sh, warp, lane, 0u, 0u};
+    bool bad = false;
     for (;;) {
-      if (threadIdx.x == 0) sh_take = atomicAdd(a.team_take, 1u);
-      __syncthreads();
-      const uint32_t k = sh_take;
-      __syncthreads();
-      if (k >= num) break;
-      cast_team(job, smem, a.team_list[k], block, slice, cap, a.deep_list, a.deep_count, bad);
+      uint32_t id = kUMax;
+      if (solo ? lane == 0 : threadIdx.x == 0) {
+        id = from_list ? atomicAdd(a.team_take, 1u) : a.parked.take_handed(sh_handed);
+        if (from_list) id = id < num ? id : kUMax;
+        else if (id != kUMax) id = links.append(num + atomicAdd(a.team_more, 1u), a.parked.work(id));
+      }
+      if (solo) {
+        id = __shfl_sync(kWarpAll, id, 0);
+        __syncwarp();
+      } else {
+        if (threadIdx.x == 0) sh_take = id;
+        __syncthreads();
+        id = sh_take;
+        __syncthreads();
+      }
+      if (id == kUMax) break;
+      if (solo) cast_team<true>(job, smem, links.work(id), one, slice, cap, id, links.next, deep, bad);
+      else cast_team<false>(job, smem, links.work(id), all, slice, cap, id, links.next, deep, bad);
     }
+    if (bad) raise_status(a.status, kStatusBadIndex);
+    __syncthreads();
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) sh_take = atomicAdd(a.done + (grouped ? 1 + group : 0), 1u);
+  __syncthreads();
+  // the last block of the group, or of all, casts what is left
+  if (sh_take != (grouped ? (gridDim.x - 1 - group) / kDeepGroups : gridDim.x - 1)) return;
+  __threadfence();
+  if (*reinterpret_cast<volatile uint32_t*>(deep) == kUMax) return;
+  if (!grouped) {
+    cast_deep(job, smem, links, deep, a.pool, a.pool_frames, static_cast<uint4*>(nullptr), 0ull, need, a.status);
   } else {
-    const Team alone{sh + warp, 0u, 1u, lane, 0u, 0u};
-    for (;;) {
-      uint32_t k = 0;
-      if (lane == 0) k = atomicAdd(a.team_take, 1u);
-      k = __shfl_sync(kWarpAll, k, 0);
-      if (k >= num) break;
-      cast_team(job, smem, a.team_list[k], alone, slice, cap, a.deep_list, a.deep_count, bad);
-    }
+    // and from the group's part of what the parked rays leave free of the first half
+    const uint64_t used = static_cast<uint64_t>(parked) * a.parked.stride, more = (half - used) / kDeepGroups;
+    cast_deep(job, smem, links, deep, a.pool + half + group * room, room, a.pool + used + group * more, more, need,
+              a.status);
   }
-  if (bad) raise_status(a.status, kStatusBadIndex);
-  // the last block casts the rays whose frames outgrew a slice (none in a tree
-  // of Morton codes, whose chains are folded), with the pool split over them,
-  // then with unbounded frames
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) sh_take = atomicAdd(a.done, 1u);
-  __syncthreads();
-  if (sh_take != gridDim.x - 1) return;
-  __threadfence();
-  const volatile uint32_t* left = a.deep_count;
-  const uint32_t n2 = left[0];
-  if (n2 == 0) return;
-  cast_deep(job, smem, a.deep_list, n2, a.last_list, a.deep_count + 1, a.pool, a.pool_frames, 0u, a.max_tri, a.status);
-  __threadfence();
-  __syncthreads();
-  const uint32_t n3 = left[1];
-  if (n3 == 0) return;
-  cast_deep(job, smem, a.last_list, n3, static_cast<uint32_t*>(nullptr), static_cast<uint32_t*>(nullptr), a.pool,
-            a.pool_frames, a.max_tri < 2 ? 2u : a.max_tri, a.max_tri, a.status);
 }
 
 // Number of resident blocks of a persistent kernel instantiation on the
@@ -1253,7 +1307,8 @@ inline uint32_t park_steps(uint32_t num_work) {
 static __global__ void k_cast_begin(uint32_t* counters) {
   pdl_wait();
   pdl_launch_dependents();
-  if (threadIdx.x < kCastCounterBytes / sizeof(uint32_t)) counters[threadIdx.x] = 0u;
+  if (threadIdx.x < kCastCounterBytes / sizeof(uint32_t))
+    counters[threadIdx.x] = threadIdx.x >= 7 && threadIdx.x < 8 + kDeepGroups ? kUMax : 0u;
 }
 
 // `busy`: the GPU has other work to do beside this cast (a server with requests
@@ -1290,31 +1345,34 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   const uint64_t room = sc.pool_bytes / 2 / (sizeof(uint4) * a.parked.stride);
   a.parked.capacity = static_cast<uint32_t>(room < (1u << 20) ? room : (1u << 20));
   a.parked_take = sc.counters + 6;
-  a.team_list = sc.list1;
+  a.links = RayLinks{sc.list1, sc.list2};
   a.team_count = sc.counters + 1;
   a.team_take = sc.counters + 4;
-  a.deep_list = sc.list2;
-  a.deep_count = sc.counters + 2;
-  a.last_list = sc.list1;
-  a.done = sc.counters + 7;
+  a.team_more = sc.counters + 2;
+  a.deep = sc.counters + 7;
+  a.done = a.deep + 1 + kDeepGroups;
   a.pool = static_cast<uint4*>(sc.pool);
   a.pool_frames = sc.pool_bytes / kFrameBytes;
   a.max_tri = max_tri;
   a.long_steps = t.cast_long_steps;
   a.status = status;
-  launch_pdl(k_cast_begin, dim3(1), dim3(32), 0, s, sc.counters);
+  const uint32_t tail_grid = 152 * kTailBlocks, group_size = (tail_grid + kDeepGroups - 1) / kDeepGroups;
+  a.slice_frames = a.pool_frames / 2 / (kDeepGroups * group_size * kTeamWarps);
+  a.group_frames = a.slice_frames * group_size * kTeamWarps;
+  launch_pdl(k_cast_begin, dim3(1), dim3(64), 0, s, sc.counters);
   launch_pdl(k_cast_persistent<Job, kThreads, kStack, !kBusy>, dim3(grid), dim3(kThreads), 0, s, job, sc.counters, sc.list1,
              sc.counters + 1, status, mins, a.parked);
-  launch_pdl(k_cast_tail<Job, kStack>, dim3(152 * kTailBlocks), dim3(kTeamThreads), 0, s, job, a);
+  launch_pdl(k_cast_tail<Job, kStack>, dim3(tail_grid), dim3(kTeamThreads), 0, s, job, a);
 }
 
 // The tiered cast of every work index of `job`: the persistent cast, then one
 // kernel for the rays it hands over (k_cast_tail).  sc.counters
-// (kCastCounterBytes) are zeroed first: [0] rays taken, [1] rays for the
-// team tier (list1), [2], [3] rays for the two deep casts (list2, list1 again),
-// [4] rays taken by the team tier, [5] rays parked, [6] parked rays taken, [7]
-// blocks done.  The first tier's block size and on-chip stack depth come from
-// the current Tuning (kCastVariants lists the choices).
+// (kCastCounterBytes) are set first: [0] rays taken, [1] rays for the team tier
+// (list1), [2] parked rays added to them, [4] rays taken by the team
+// tier, [5] rays parked, [6] parked rays taken, from [7] on the lists of rays with
+// more frames (linked by list2), of all blocks and of each group, then the blocks
+// done likewise.  The first tier's block size and on-chip stack depth come from the
+// current Tuning (kCastVariants lists the choices).
 template <typename Job, bool kBusy = false>
 inline void cast_job(cudaStream_t s, const Job& job, const CastScratch& sc, uint32_t max_tri, uint32_t* status) {
   if (job.num_work == 0) return;

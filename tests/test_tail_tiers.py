@@ -58,3 +58,53 @@ def test_chain_left_at_every_link(cuda, oracle, n, repeat):
     assert np.array_equal(r_hit, np.repeat(np.arange(n, dtype=np.uint32), repeat))
     assert np.array_equal(hit, r_hit)
     assert np.array_equal(bits(t), bits(r_t))
+
+
+def _comb(T):
+    """A brought tree whose every branch has a leaf on the right and the rest, which is
+    nearer to rays that come from below, on the left: a ray through all boxes has a
+    frame on each level, and no chain to fold.  The nearer a triangle, the smaller, so
+    that rays further out pop frames whose leaves they hit."""
+    z = (T - np.arange(T)) / T
+    size = 0.2 + np.round(50 * z) / 50
+    vtx = np.zeros((T, 3, 3), np.float32)
+    vtx[:, :, :2] = size[:, None, None] * np.array([[-2, -2], [4, -2], [-2, 4]])
+    vtx[:, :, 2] = z[:, None]
+    tri = np.arange(3 * T, dtype=np.uint32).reshape(-1, 3)
+    i = np.arange(T - 1)
+    bvh = np.full((2 * T - 1, 3), 0xFFFFFFFF, np.uint32)
+    bvh[1:T - 1, 0] = i[:-1]
+    bvh[:T - 1, 1] = np.where(i < T - 2, i + 1, 2 * T - 2)
+    bvh[:T - 1, 2] = T - 1 + i
+    bvh[T - 1:, 0] = np.minimum(np.arange(T), T - 2)
+    bvh[T - 1:, 1] = np.arange(T)
+    aabb = np.empty((2 * T - 1, 6), np.float32)
+    aabb[:, :2], aabb[:, 3:5] = -4.0, 8.0  # every ray meets every box
+    aabb[T - 1:, 2] = aabb[T - 1:, 5] = z
+    aabb[:T - 1, 2], aabb[:T - 1, 5] = z[-1], z[:T - 1]
+    org = np.random.default_rng(T).uniform(-1.0, 1.0, (20_000, 3)).astype(np.float32)
+    org[:, 2] = -1.0
+    return tri, vtx.reshape(-1, 3), bvh, aabb, org, np.tile(np.float32([0, 0, 1]), (20_000, 1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,num_ray", [(60, 3000), (500, 3000), (1300, 3000), (1300, 20_000), (5000, 300),
+                                       (30_000, 300), (100_000, 60)])
+def test_trees_deeper_than_a_stack(cuda, oracle, T, num_ray):
+    """Within the on-chip stack, a team's slice, and with stacks carved from a group's
+    share of the pool or (from 14,600 levels on) from the whole."""
+    tri, vtx, bvh, aabb, org, d = _comb(T)
+    org, d = org[:num_ray], d[:num_ray]
+    hit, t, c = _cast(cuda, tri, vtx, bvh, aabb, org, d)
+    assert c[5] > 0  # parked
+    assert (c[7:32] == 0xFFFFFFFF).all()  # the lists of rays handed on are empty again
+    # the last, nearest triangle that holds the ray's point
+    near = np.full(num_ray, 0xFFFFFFFF, np.uint32)
+    for k in range(T):
+        s = vtx[3 * k + 1, 0] / 4
+        near[(org[:, 0] > -2 * s) & (org[:, 1] > -2 * s) & (org[:, 0] + org[:, 1] < 2 * s)] = k
+    assert np.array_equal(hit, near)
+    if T <= 5000:
+        r_hit, r_t = oracle.cast_rays(org, d, tri, vtx, bvh, aabb)
+        assert np.array_equal(hit, r_hit)
+        assert np.array_equal(bits(t), bits(r_t))
