@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kThreads) k_centroid_aabb(uint32_t num_tri, co
 template <bool kHist>
 __global__ void __launch_bounds__(kThreads) k_morton_tri(uint32_t num_tri, const uint32_t* __restrict__ tri2vtx,
                                                         uint32_t num_vtx, const float* __restrict__ vtx2xyz,
-                                                        const float* __restrict__ transform,
+                                                        const float* transform,
                                                         uint32_t* __restrict__ codes, uint32_t* __restrict__ hist,
                                                         uint32_t* status, const float* cent, size_t stride,
                                                         bool hist10) {
@@ -310,9 +310,8 @@ __global__ void __launch_bounds__(kThreads) k_vtx2morton(uint32_t n, uint32_t nu
 // ----------------------------------------------------------------- topology
 
 template <int kTh>
-__global__ void __launch_bounds__(kTh) k_topology(uint32_t n, const uint32_t* __restrict__ c,
-                                                 const uint32_t* __restrict__ idx2obj, uint32_t* bvhnodes,
-                                                 uint32_t* other_end, uint32_t* flags, uint32_t* hdr) {
+__global__ void __launch_bounds__(kTh) k_topology(uint32_t n, const uint32_t* c, const uint32_t* idx2obj,
+                                                 uint32_t* bvhnodes, uint32_t* other_end, uint32_t* flags, uint32_t* hdr) {
   const uint32_t ib = blockIdx.x * kTh + threadIdx.x;
   if (flags) {  // idle since before the predecessor, which does not touch them
     if (ib < n) flags[ib] = 0u;
@@ -1543,6 +1542,11 @@ void launch_refit(cudaStream_t s, uint32_t num_tri, const uint32_t* bvhnodes, co
   // gated, it usually exits at once: a grid of a few blocks per SM costs
   // less to launch than one thread per leaf
   if (gate != nullptr && grid > 152u * 8u) grid = 152u * 8u;
+  if (gate == nullptr) {  // the tree is the first that it reads, and read-only: a normal launch
+    k_refit<<<grid, kThreads, 0, s>>>(num_tri, bvhnodes, tri2vtx, num_vtx, vtx2xyz0, vtx2xyz1, aabb, flags, height_out,
+                                      status, gate);
+    return;
+  }
   launch_pdl(k_refit, dim3(grid), dim3(kThreads), 0, s, num_tri, bvhnodes, tri2vtx, num_vtx, vtx2xyz0, vtx2xyz1, aabb,
              flags, height_out, status, gate);
 }

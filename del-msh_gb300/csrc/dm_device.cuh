@@ -24,11 +24,19 @@ enum DeviceStatusBits : uint32_t {
 // Programmatic dependent launch.  A kernel launched with
 // launch_pdl (dm_internal.h) may start while its predecessor in the stream
 // is still running; pdl_wait() returns once the predecessor has completed
-// and its writes are visible (at once for a normal launch).  Each such
-// kernel calls pdl_launch_dependents() only after pdl_wait(), so when the
-// next kernel starts early every kernel before this one has completed: code
-// before pdl_wait() may read results of those, but nothing this kernel's
-// predecessor writes, and may write nothing that it reads.
+// and its writes are visible (at once for a normal launch).  A kernel calls
+// pdl_launch_dependents() only when all before it have completed: after its own
+// pdl_wait(), or at any time if it is always launched normally (k_refit_begin, the
+// clusters of k_batch_seg_build).  So when the next kernel starts early every kernel
+// but its predecessor has completed: code before pdl_wait() may read results of
+// those, but nothing this kernel's predecessor writes, and may write nothing that
+// it reads.  (The one exception: k_batch_seg_build<1> does all its work beside
+// the clusters, on other meshes, taken from a cursor that both advance by atomics,
+// and waits at its end.)
+// Read-only loads (__ldg, or through a const __restrict__ parameter) of what the
+// predecessor writes may be moved ahead of the wait, as nothing says that they
+// depend on it: they have to be ordinary loads, unless their address, or a branch
+// before them, depends on a value read after the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -6,14 +6,16 @@
 namespace dm {
 
 // Code / object accessors: the single-mesh arrays, or a segment of the
-// batched sort's (mesh << 30 | code) keys and global triangle indices.
+// batched sort's (mesh << 30 | code) keys and global triangle indices.  Ordinary
+// loads: k_topology starts while the sort that writes the arrays still runs (see
+// pdl_wait).
 struct Codes32 {
   const uint32_t* p;
-  __device__ __forceinline__ uint32_t operator()(uint32_t i) const { return __ldg(p + i); }
+  __device__ __forceinline__ uint32_t operator()(uint32_t i) const { return p[i]; }
 };
 struct Objs32 {
   const uint32_t* p;
-  __device__ __forceinline__ uint32_t operator()(uint32_t i) const { return __ldg(p + i); }
+  __device__ __forceinline__ uint32_t operator()(uint32_t i) const { return p[i]; }
 };
 
 // Last index of the run of value v that contains position `from` (sorted c).
@@ -104,26 +106,28 @@ __device__ __forceinline__ void topology_node(uint32_t n, const Codes& c, const 
                                               uint32_t ib, uint32_t* other_end) {
   uint32_t r0, r1, isplit;
   karras_range_split(n, c, ib, r0, r1, isplit);
+  const bool leaf0 = r0 == isplit, leaf1 = r1 == isplit + 1;
+  const uint32_t obj0 = leaf0 ? obj(isplit) : 0u, obj1 = leaf1 ? obj(isplit + 1) : 0u;
   if (other_end) other_end[ib] = (r0 == ib) ? r1 : r0;
   const uint32_t nb = n - 1;
   uint32_t* me = bvhnodes + static_cast<size_t>(ib) * 3;
-  if (r0 == isplit) {
+  if (leaf0) {
     const uint32_t a = nb + isplit;
     me[1] = a;
     uint32_t* la = bvhnodes + static_cast<size_t>(a) * 3;
     la[0] = ib;
-    la[1] = obj(isplit);
+    la[1] = obj0;
     la[2] = kUMax;
   } else {
     me[1] = isplit;
     bvhnodes[static_cast<size_t>(isplit) * 3] = ib;
   }
-  if (r1 == isplit + 1) {
+  if (leaf1) {
     const uint32_t b = nb + isplit + 1;
     me[2] = b;
     uint32_t* lb = bvhnodes + static_cast<size_t>(b) * 3;
     lb[0] = ib;
-    lb[1] = obj(isplit + 1);
+    lb[1] = obj1;
     lb[2] = kUMax;
   } else {
     me[2] = isplit + 1;

@@ -76,7 +76,7 @@ template <typename KeyT, bool kIota, int kWindow>
 __global__ void __launch_bounds__(kThreads, sizeof(KeyT) == 4 ? 4 : 2) k_onesweep(const KeyT* __restrict__ keys_in,
                                                       const uint32_t* __restrict__ vals_in, KeyT* __restrict__ keys_out,
                                                       uint32_t* __restrict__ vals_out, uint32_t n, uint32_t shift,
-                                                      const uint32_t* __restrict__ hist, uint32_t* lookback,
+                                                      const uint32_t* hist, uint32_t* lookback,
                                                       uint32_t* tile_counter, uint32_t* status,
                                                       uint32_t spin_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(KeyT) == 4 ? 4 : 2) k_oneswee
   if (tid == 0) S.tile = atomicAdd(tile_counter, 1u);
   pdl_wait();
   pdl_launch_dependents();
-  const uint32_t gb = block_exclusive_scan(__ldg(hist + tid), S.scan);  // has __syncthreads
+  const uint32_t gb = block_exclusive_scan(hist[tid], S.scan);  // has __syncthreads
   S.gbase[tid] = gb;
   const uint32_t tile = S.tile;
   const uint32_t tile_base = tile * kSortTile;
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kThreadsM, 3) k_onesweep_match(const uint32_t*
                                                                const uint32_t* __restrict__ vals_in,
                                                                uint32_t* __restrict__ keys_out,
                                                                uint32_t* __restrict__ vals_out, uint32_t n,
-                                                               uint32_t shift, const uint32_t* __restrict__ hist,
+                                                               uint32_t shift, const uint32_t* hist,
                                                                uint32_t* lookback, uint32_t* tile_counter,
                                                                uint32_t* status, uint32_t spin_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kThreadsM, 3) k_onesweep_match(const uint32_t*
     keys[j] = idx < n ? keys_in[idx] : 0u;
   }
   // the keys are on their way during the scan of the upfront histogram
-  const uint32_t gb = block_exclusive_scan_m(tid < kRadix ? __ldg(hist + tid) : 0u, S.scan);  // has __syncthreads
+  const uint32_t gb = block_exclusive_scan_m(tid < kRadix ? hist[tid] : 0u, S.scan);  // has __syncthreads
   if (tid < kRadix) S.gbase[tid] = gb;
   // Rank inside the warp in (j, lane) order, i.e. input order.
   const uint32_t lt_mask = (1u << lane) - 1u;
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep10(const uint32_t* __re
                                                           const uint32_t* __restrict__ vals_in,
                                                           uint32_t* __restrict__ keys_out,
                                                           uint32_t* __restrict__ vals_out, uint32_t n, uint32_t shift,
-                                                          const uint32_t* __restrict__ hist, uint32_t* lookback,
+                                                          const uint32_t* hist, uint32_t* lookback,
                                                           uint32_t* tile_counter, uint32_t* status,
                                                           uint32_t spin_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_onesweep10(const uint32_t* __re
   pdl_wait();
   pdl_launch_dependents();
   // global start of digits 4*tid .. 4*tid+3 (scan of the upfront histogram)
-  const uint4 h4 = __ldg(reinterpret_cast<const uint4*>(hist) + tid);
+  const uint4 h4 = reinterpret_cast<const uint4*>(hist)[tid];
   const uint32_t hsum = h4.x + h4.y + h4.z + h4.w;
   {
     const uint32_t base = block_exclusive_scan(hsum, S.scan);  // has __syncthreads
