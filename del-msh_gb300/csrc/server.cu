@@ -135,7 +135,6 @@ struct Slot {
   size_t build_bytes = 0;
   void* cast_scratch = nullptr;
   size_t cast_bytes = 0;
-  float* d_transform = nullptr;
   float* d_rays = nullptr;  // max_out origins then max_out directions
   uint32_t* d_hit = nullptr;
   float* d_t = nullptr;
@@ -472,7 +471,6 @@ int dm_server_create(int device, size_t budget_bytes, int num_slots, uint32_t ma
         cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) != cudaSuccess ||
         cudaMalloc(&sl.build_scratch, sl.build_bytes) != cudaSuccess ||
         cudaMalloc(&sl.cast_scratch, sl.cast_bytes) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&sl.d_transform), 64) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&sl.d_rays), 24ull * max_out) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&sl.d_hit), 4ull * max_out) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&sl.d_t), 4ull * max_out) != cudaSuccess) {
@@ -640,7 +638,6 @@ int dm_server_destroy(dm_server* S) {
   for (auto& sl : S->slots) {
     cudaFree(sl.build_scratch);
     cudaFree(sl.cast_scratch);
-    cudaFree(sl.d_transform);
     cudaFree(sl.d_rays);
     cudaFree(sl.d_hit);
     cudaFree(sl.d_t);
