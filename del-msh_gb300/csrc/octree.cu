@@ -280,7 +280,9 @@ __global__ void __launch_bounds__(kThreads) k_make_tree(uint32_t num_idx, const 
 // does not matter for the result, only for how early the paths meet.
 
 // Peers' values summed into the lowest lane of each group (all lanes of
-// `members` call it; `peers` are the lanes of the caller's group).
+// `members` call it; `peers` are the lanes of the caller's group).  The published
+// peer reduction of E. Westphal, "Voting and Shuffling to Optimize Atomic
+// Operations" (2015): each lane adds the next peer's value, the odd ranks drop out.
 template <int kV>
 __device__ __forceinline__ void sum_peers(uint32_t members, uint32_t peers, uint32_t lane, float (&v)[kV]) {
   uint32_t rank = __popc(peers & ((1u << lane) - 1u));
