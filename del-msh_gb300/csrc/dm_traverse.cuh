@@ -401,7 +401,7 @@ constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 // of the warp wait for it, or when nothing else can run.
 struct PhaseMins {
   uint32_t refill, leaf, ascend;
-  uint32_t long_steps;  // node entries after which a ray at a long chain goes to the team tier
+  uint32_t long_steps;  // node entries after which a ray is handed to the team tier
   uint32_t park_steps;  // node entries after which a ray is parked for the split tier
   uint32_t share;       // rays a warp takes at a time, at most
 };
@@ -1296,19 +1296,10 @@ inline int persistent_grid() {
 // smoothest two of the six, 1920 x 1080 takes 485 and 497 us against 465 and 467.
 constexpr uint32_t kParkSteps = 24, kParkRays = 16384, kParkMore = 14, kParkDoublings = 5;
 
-// In a tree of up to kParkSmallTri triangles no ray goes on for much longer than
-// kParkSmallSteps, and the tail costs more than it saves.  Parked from 24 / from 64
-// entries: 20,000 rays on 80 triangles 50.5 / 41.4 us, on 200 61.9 / 51.7, on 648
-// 70.5 / 64.0; 64 x 64 pixels of 200 triangles 45.6 / 37.5, of 648 49.7 / 41.4.  Beyond
-// that the lower threshold wins: 1,000 and 20,000 rays on 1,250 triangles 52.5 / 57.8
-// and 79.1 / 85.3, on 2,048 53.7 / 61.9 and 78.3 / 88.5.
-constexpr uint32_t kParkSmallTri = 1024, kParkSmallSteps = 64;
-
-inline uint32_t park_steps(uint32_t num_work, uint32_t max_tri) {
+inline uint32_t park_steps(uint32_t num_work) {
   uint32_t doublings = 0;
   for (uint32_t n = num_work; n >= 2 * kParkRays && doublings < kParkDoublings; n >>= 1) ++doublings;
-  const uint32_t steps = kParkSteps + kParkMore * doublings;
-  return max_tri <= kParkSmallTri && steps < kParkSmallSteps ? kParkSmallSteps : steps;
+  return kParkSteps + kParkMore * doublings;
 }
 
 // Zeroes a cast's counters.  A kernel instead of a copy-engine memset, so that
@@ -1345,15 +1336,8 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   // (at 9, 8, 6 for a mesh and 13, 12, 9 for the batch: 437, 438, 441; 1230,
   // 1231, 1253 us).
   const uint32_t refill = min(t.cast_refill_min * Job::kRefillHalves / 2u, 32u);
-  const uint32_t park = kBusy ? kUMax : park_steps(job.num_work, max_tri);
-  // A ray that would be parked at a long chain goes to the team tier at once.  Parked, it
-  // got there only by the split tier's block, behind that block's other rays, and was cast
-  // by it alone.  Rays on clustered soups, parked / handed over: 10,000 on 20 thousand
-  // triangles 91 / 95 us, on 70 thousand 189 / 163, on 200 thousand 228 / 195, on 1
-  // million 310 / 214, on 4 million 472 / 287; 60,000 on 200 thousand 304 / 230, on 4
-  // million 640 / 457.  (With the lower bound in the split tier too: 60,000 on 20 and 70
-  // thousand 199 and 220 us, 140 and 162 so.)
-  const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, min(t.cast_long_steps, park), park, share};
+  const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps,
+                       kBusy ? kUMax : park_steps(job.num_work), share};
   TailArgs a;
   a.parked.rays = static_cast<uint4*>(sc.pool);
   a.parked.count = sc.counters + 5;
