@@ -1296,10 +1296,19 @@ inline int persistent_grid() {
 // smoothest two of the six, 1920 x 1080 takes 485 and 497 us against 465 and 467.
 constexpr uint32_t kParkSteps = 24, kParkRays = 16384, kParkMore = 14, kParkDoublings = 5;
 
-inline uint32_t park_steps(uint32_t num_work) {
+// In a tree of up to kParkSmallTri triangles no ray goes on for much longer than
+// kParkSmallSteps, and the tail costs more than it saves.  Parked from 24 / from 64
+// entries: 20,000 rays on 80 triangles 50.5 / 41.4 us, on 200 61.9 / 51.7, on 648
+// 70.5 / 64.0; 64 x 64 pixels of 200 triangles 45.6 / 37.5, of 648 49.7 / 41.4.  Beyond
+// that the lower threshold wins: 1,000 and 20,000 rays on 1,250 triangles 52.5 / 57.8
+// and 79.1 / 85.3, on 2,048 53.7 / 61.9 and 78.3 / 88.5.
+constexpr uint32_t kParkSmallTri = 1024, kParkSmallSteps = 64;
+
+inline uint32_t park_steps(uint32_t num_work, uint32_t max_tri) {
   uint32_t doublings = 0;
   for (uint32_t n = num_work; n >= 2 * kParkRays && doublings < kParkDoublings; n >>= 1) ++doublings;
-  return kParkSteps + kParkMore * doublings;
+  const uint32_t steps = kParkSteps + kParkMore * doublings;
+  return max_tri <= kParkSmallTri && steps < kParkSmallSteps ? kParkSmallSteps : steps;
 }
 
 // Zeroes a cast's counters.  A kernel instead of a copy-engine memset, so that
@@ -1336,8 +1345,8 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   // (at 9, 8, 6 for a mesh and 13, 12, 9 for the batch: 437, 438, 441; 1230,
   // 1231, 1253 us).
   const uint32_t refill = min(t.cast_refill_min * Job::kRefillHalves / 2u, 32u);
-  const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps,
-                       kBusy ? kUMax : park_steps(job.num_work), share};
+  const uint32_t park = kBusy ? kUMax : park_steps(job.num_work, max_tri);
+  const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps, park, share};
   TailArgs a;
   a.parked.rays = static_cast<uint4*>(sc.pool);
   a.parked.count = sc.counters + 5;
