@@ -401,7 +401,7 @@ constexpr int kDeepRing = 64;  // on-chip frames per ray of the overflow tiers
 // of the warp wait for it, or when nothing else can run.
 struct PhaseMins {
   uint32_t refill, leaf, ascend;
-  uint32_t long_steps;  // node entries after which a ray is handed to the team tier
+  uint32_t long_steps;  // node entries after which a ray at a long chain goes to the team tier
   uint32_t park_steps;  // node entries after which a ray is parked for the split tier
   uint32_t share;       // rays a warp takes at a time, at most
 };
@@ -1346,7 +1346,14 @@ inline void launch_tiers(cudaStream_t s, const Job& job, const CastScratch& sc, 
   // 1231, 1253 us).
   const uint32_t refill = min(t.cast_refill_min * Job::kRefillHalves / 2u, 32u);
   const uint32_t park = kBusy ? kUMax : park_steps(job.num_work, max_tri);
-  const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, t.cast_long_steps, park, share};
+  // A ray that would be parked at a long chain goes to the team tier at once.  Parked, it
+  // got there only by the split tier's block, behind that block's other rays, and was cast
+  // by it alone.  Rays on clustered soups, parked / handed over: 10,000 on 20 thousand
+  // triangles 91 / 95 us, on 70 thousand 189 / 163, on 200 thousand 228 / 195, on 1
+  // million 310 / 214, on 4 million 472 / 287; 60,000 on 200 thousand 304 / 230, on 4
+  // million 640 / 457.  (With the lower bound in the split tier too: 60,000 on 20 and 70
+  // thousand 199 and 220 us, 140 and 162 so.)
+  const PhaseMins mins{refill, t.cast_leaf_min, t.cast_ascend_min, min(t.cast_long_steps, park), park, share};
   TailArgs a;
   a.parked.rays = static_cast<uint4*>(sc.pool);
   a.parked.count = sc.counters + 5;

@@ -86,9 +86,10 @@ typedef struct dm_tuning {
   uint32_t cast_leaf_min;
   uint32_t cast_ascend_min;
   /* Node entries after which the persistent cast, once a warp has no more
-     rays to take, hands a ray entering a long run of chain links to the warp
-     tier, where one warp runs it and folds the links 32 at a time: 1..2^30,
-     0 = the default (64).  Results do not depend on it. */
+     rays to take, hands a ray entering a long run of chain links to the team
+     tier, where a team of warps runs it and folds the links: 1..2^30, 0 = the
+     default (64).  A lower bound holds where rays are parked for the split
+     tier after fewer entries.  Results do not depend on it. */
   uint32_t cast_long_steps;
   /* Batched build: 0 = every mesh sorted and linked on chip when the largest
      has at most 65536 triangles (else the global sort), 1 = the global 64-bit
